@@ -305,10 +305,10 @@ def work(case):
             b, f = b + x * case["steps"], f + y * case["steps"]
         return {"bytes": b, "flops": f}
     if kind == "cavity":
-        # the pressure solve's Krylov steps (about 2.5 n of them, 500 at most) each need the basis so far once;
+        # the pressure solve's Krylov steps (about 4 n of them, 500 at most) each need the basis so far once;
         # the momentum solves take a handful
         cells = case["n"] ** 2 * (2 if case["triangles"] else 1)
-        k = min(500, round(2.5 * case["n"]))
+        k = min(500, 4 * case["n"])
         return {"bytes": float(8 * cells * (k * (k + 1) / 2 + 12 * k)) * case["inner"],
                 "flops": float(cells * (4 * k * (k + 1) / 2 + 14 * k)) * case["inner"]}
     macs = sum(k * n for k, n in _layers(case))
