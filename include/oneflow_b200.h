@@ -345,10 +345,11 @@ typedef struct ofg_tuning {
     int    grad_min_blocks;   /* gradients + limiter: 4, 6 (default) or 8          */
     int    sweep_min_blocks;  /* LU-SGS level kernels: 6, 8 (default) or 10        */
     int    sweep_block;       /* LU-SGS level kernels: 64 or 128 (default)         */
-    int    sweep_persistent;  /* 0: one launch per level (default); 1: one launch
-                                 per sweep, a single block running every level
-                                 with a block barrier between levels (the same
-                                 bits; for many small levels).  Both paths.   */
+    int    sweep_persistent;  /* 0: one launch per level; 1: one launch per sweep,
+                                 one cluster of blocks chaining the levels (the
+                                 same bits; for many small levels).  Both paths.
+                                 Until set or tuned, ofg_upload_mesh chooses by
+                                 the mesh's levels.                           */
     int    grad_block;        /* gradients + limiter threads per block: 64 or 128
                                  (default; 0 also means 128)                  */
     int    reserved[1];

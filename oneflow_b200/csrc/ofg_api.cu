@@ -37,10 +37,20 @@ int launch(ofg_ctx *c, int task) {
     return OFG_OK;
 }
 
+bool has_turb(const ofg_ctx *c) { return c->p.vismodel >= 3; }
+bool multi_stage(const ofg_ctx *c) { return c->p.time_integral == 1; }
+
+// after a synchronisation: an error if a chained sweep's wait ran out (the flag is cleared)
+int chain_status(ofg_ctx *c) {
+    if (!c->chainStatus || !*static_cast<volatile unsigned *>(c->chainStatus)) return OFG_OK;
+    *static_cast<volatile unsigned *>(c->chainStatus) = 0;
+    return c->fail(OFG_E_TIMEOUT, "a chained sweep's wait ran out");
+}
+
 int sync(ofg_ctx *c) {
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return c->fail(OFG_E_CUDA, std::string("stream: ") + cudaGetErrorString(e));
-    return OFG_OK;
+    return chain_status(c);
 }
 
 // ---------------------------------------------------------------------------
@@ -249,6 +259,28 @@ void build_levels(ofg_ctx *c, bool lower, std::vector<int> &order, std::vector<i
     for (int k = 0; k < N; ++k) { int i = c->keyOrder[k]; order[pos[lev[i]]++] = i; }
 }
 
+// Whether the chained sweeps (ofg_chain.cuh) pay on this mesh: many levels,
+// each small enough for one cluster.  Measured, us a lower sweep, one launch
+// per level against the chain: 119 levels of 29 cells 785-950 / 83; 385 of 170
+// 3,130 / 430; 301 of 325 (wing, mixed) 2,360 / 1,270; 228 of 631 2,320 / 1,190;
+// 398 of 1,809 (mixed) 3,230 / 3,780, the chain no longer faster.  With two
+// levels of 2,048 cells the launches win, 15 / 32.
+bool chain_pays(const ofg_ctx *c) {
+    const int nlev = std::max<int>(1, int(c->lowOff.size()) - 1);
+    return nlev >= 16 && c->nCells / nlev <= 1024;
+}
+
+void free_chain(ofg_ctx *c) {
+    for (ChainBuf &b : c->chain) {
+        for (int *p : {b.lev, b.ref, b.edge, b.cell}) cudaFree(p);
+        b = ChainBuf();
+    }
+    cudaFree(c->d_chainCoef);
+    cudaFree(c->d_chainCell);
+    c->d_chainCoef = nullptr;
+    c->d_chainCell = nullptr;
+}
+
 // Per-cell neighbour lists in ascending face id (the c2f order), one int2 per
 // face: {face | side << 31, neighbour}, side = 1 where the cell is the face's
 // right cell.  Full lists for the residual and gradient gathers; for the
@@ -279,6 +311,85 @@ void build_lists(const ofg_ctx *c, NbLists &L) {
         L.loOff[i + 1] = int(L.lol.size() / 2);
         L.upOff[i + 1] = int(L.upl.size() / 2);
     }
+}
+
+template <typename T> int upload(ofg_ctx *c, T **d, const T *h, size_t n);
+int upload_bytes(ofg_ctx *c, void **d, const void *h, size_t bytes);
+
+// The chained sweeps' schedules (ofg_chain.cuh): edge slots [level][j-th edge][cell of the level], each edge with
+// its neighbour's place in the ring, or ~neighbour where the ring no longer (or not for the whole level) holds it.
+// Without the memory for them, or where a level is wider than the cluster's
+// signals can carry, the sweeps stay one launch per level.
+int build_chain(ofg_ctx *c, const NbLists *lists = nullptr) {
+    if (c->chain[0].lev) return OFG_OK;
+    if (!c->chainStatus) {
+        CK(cudaHostAlloc((void **)&c->chainStatus, sizeof(unsigned), cudaHostAllocDefault));
+        *c->chainStatus = 0;
+    }
+    NbLists own;
+    if (!lists) {
+        build_lists(c, own);
+        lists = &own;
+    }
+    long long most = 1;
+    std::vector<int> lev, ref, edge, cell, pos(c->nCells), at(c->nCells);
+    for (int dir = 0; dir < 2; ++dir) {
+        const std::vector<int> &order = dir == 0 ? c->lowOrder : c->upOrder, &off = dir == 0 ? c->lowOff : c->upOff;
+        const std::vector<int> &nbOff = dir == 0 ? lists->loOff : lists->upOff;
+        const std::vector<int> &nbl = dir == 0 ? lists->lol : lists->upl;
+        const int nlev = int(off.size()) - 1;
+        lev.assign(4 * (size_t)nlev, 0);
+        long long slots = 0;
+        for (int l = 0; l < nlev; ++l) {
+            int deg = 0;
+            for (int k = off[l]; k < off[l + 1]; ++k) {
+                const int i = order[k];
+                pos[i] = k; at[i] = l;
+                deg = std::max(deg, nbOff[i + 1] - nbOff[i]);
+            }
+            int *m = &lev[4 * (size_t)l];
+            m[0] = off[l]; m[1] = off[l + 1] - off[l]; m[2] = int(slots); m[3] = deg;
+            slots += (long long)deg * m[1];
+            if (slots > INT32_MAX || m[1] > kChainLevel) { free_chain(c); return OFG_OK; }
+        }
+        ref.assign(slots, kChainNone); edge.assign(2 * slots, -1); cell.assign(slots, 0);
+        int far = 0;
+        for (int l = 0; l < nlev; ++l) {
+            const int *m = &lev[4 * (size_t)l];
+            for (int t = 0; t < m[1]; ++t) {
+                const int i = order[m[0] + t];
+                size_t s = (size_t)m[2] + t;
+                for (int q = nbOff[i]; q < nbOff[i + 1]; ++q, s += m[1]) {   // ascending face id
+                    const int nb = nbl[2 * (size_t)q + 1];
+                    const bool near = pos[nb] + kChainRing >= off[l + 1];
+                    ref[s] = near ? pos[nb] & (kChainRing - 1) : ~nb;
+                    // a global copy written after its signal is safe to read
+                    // from the level after its warp's next signal on
+                    if (!near) far = std::max(far, l <= at[nb] + kChainGroups ? 2 : 1);
+                    edge[2 * s] = nbl[2 * (size_t)q];
+                    edge[2 * s + 1] = nb;
+                    cell[s] = i;
+                }
+            }
+        }
+        ChainBuf &b = c->chain[dir];
+        b.nlev = nlev; b.slots = slots; b.far = far;
+        most = std::max(most, slots);
+        int rc = upload(c, &b.lev, lev.data(), lev.size());
+        if (!rc) rc = upload(c, &b.ref, ref.data(), ref.size());
+        if (!rc) rc = upload(c, &b.edge, edge.data(), edge.size());
+        if (!rc) rc = upload(c, &b.cell, cell.data(), cell.size());
+        if (!rc && dir == 1)
+            rc = upload_bytes(c, &c->d_chainCoef, nullptr, (size_t)most * kEdgeCoefs *
+                              (c->p.precision == OFG_PREC_MIXED ? sizeof(float) : sizeof(double)));
+        if (!rc && dir == 1) rc = upload(c, &c->d_chainCell, (const double *)nullptr, (size_t)kChainCell * c->nCells);
+        if (rc) {
+            cudaGetLastError();
+            free_chain(c);
+            return OFG_OK;
+        }
+    }
+    return OFG_OK;
 }
 
 // face records [F][8] (nx ny nz area xfc yfc zfc dist) and cell records [nT][4]
@@ -364,8 +475,6 @@ double host_sutherland(const DevParams &P, double t) {
     return std::sqrt(t3) * (1 + P.sutherland_ts) / (t + P.sutherland_ts);
 }
 
-bool has_turb(const ofg_ctx *c) { return c->p.vismodel >= 3; }
-bool multi_stage(const ofg_ctx *c) { return c->p.time_integral == 1; }
 
 int check_tid(ofg_ctx *c, int tid) {
     if (!c) return OFG_E_ARG;
@@ -435,11 +544,13 @@ void ofg_destroy(ofg_ctx *c) {
     destroy_graphs(c);
     void *ptrs[] = {c->d_lcb, c->d_bct, c->d_nb_off, c->d_nbl, c->d_lo_off, c->d_lol, c->d_up_off, c->d_upl,
                     c->d_lowOrder, c->d_upOrder, c->d_key, c->d_fgeo, c->d_cgeo, c->d_wdist, c->d_wall, c->d_wallG,
-                    c->d_fgeoD, c->d_fofs, c->d_lr, c->d_fout, c->d_lowOff, c->d_upOff,
+                    c->d_fgeoD, c->d_fofs, c->d_lr, c->d_fout,
                     c->d_q[0], c->d_q[1], c->d_qs[0], c->d_qs[1], c->d_res, c->d_dq, c->d_dt, c->d_invsr, c->d_vissr, c->d_rad,
                     c->d_bcq, c->d_partial, c->d_npart, c->d_tpart, c->d_red, c->d_redCount, c->d_stage, c->d_scal, c->d_hist, c->d_gl, c->d_mm, c->d_fix,
                     c->d_nut, c->d_dnut, c->d_resT, c->d_impsrT, c->d_matL, c->d_matR, c->d_thist, c->d_gnut};
     for (void *v : ptrs) if (v) cudaFree(v);
+    free_chain(c);
+    if (c->chainStatus) cudaFreeHost(c->chainStatus);
     cudaStreamDestroy(c->ownStream ? c->ownStream : c->stream);
     delete c;
 }
@@ -526,6 +637,9 @@ int ofg_upload_mesh(ofg_ctx *c, int nNodes, const double *xN, const double *yN, 
         if ((rc = upload(c, &c->d_lol, L.lol.data(), L.lol.size()))) return rc;
         if ((rc = upload(c, &c->d_up_off, L.upOff.data(), L.upOff.size()))) return rc;
         if ((rc = upload(c, &c->d_upl, L.upl.data(), L.upl.size()))) return rc;
+        free_chain(c);
+        if (!c->tuneSet) c->tune.sweep_persistent = chain_pays(c) ? 1 : 0;
+        if (c->tune.sweep_persistent && !multi_stage(c) && (rc = build_chain(c, &L))) return rc;
     }
     // metrics on the GPU (UnsGrid::CalcMetrics); for an SA solve without a
     // caller-supplied wall distance, CALC_WALL_DIST on the GPU as well
@@ -540,8 +654,6 @@ int ofg_upload_mesh(ofg_ctx *c, int nNodes, const double *xN, const double *yN, 
     if ((rc = upload(c, &c->d_bct, c->bct.data(), nBFaces))) return rc;
     if ((rc = upload(c, &c->d_lowOrder, c->lowOrder.data(), nCells))) return rc;
     if ((rc = upload(c, &c->d_upOrder, c->upOrder.data(), nCells))) return rc;
-    if ((rc = upload(c, &c->d_lowOff, c->lowOff.data(), c->lowOff.size()))) return rc;
-    if ((rc = upload(c, &c->d_upOff, c->upOff.data(), c->upOff.size()))) return rc;
     if ((rc = upload(c, &c->d_key, c->key.data(), c->nT))) return rc;
     if ((rc = upload(c, &c->d_wdist, c->wdist.data(), nCells))) return rc;
     {
@@ -1145,7 +1257,8 @@ int ofg_batch_step(ofg_batch *b, int nsteps) {
     float ms = 0.f;
     if (cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]) != cudaSuccess) return b->fail(OFG_E_CUDA, "cudaEventElapsedTime");
     for (int i = 0; i < n; ++i) {
-        int rc = sync_history(b->ctx[i]);
+        int rc = chain_status(b->ctx[i]);
+        if (!rc) rc = sync_history(b->ctx[i]);
         if (rc) return b->fail(rc, "context " + std::to_string(i) + ": " + b->ctx[i]->err);
     }
     b->lastMs = ms;
@@ -1562,6 +1675,8 @@ int ofg_set_tuning(ofg_ctx *c, const ofg_tuning *t) {
     ofg_tuning n = *t;
     n.ms_default = c->tune.ms_default; n.ms_tuned = c->tune.ms_tuned;
     c->tune = n;
+    c->tuneSet = true;
+    if (n.sweep_persistent && c->haveMesh && (rc = build_chain(c))) return rc;
     destroy_graphs(c);   // recaptured with the new kernels at the next ofg_step
     return OFG_OK;
 }
@@ -1636,12 +1751,14 @@ int ofg_autotune(ofg_ctx *c, int reps, ofg_tuning *out) {
         groups.push_back({&T.sweep_min_blocks, &T.sweep_block,
                           {{6, 128}, {8, 128}, {10, 128}, {6, 64}, {8, 64}, {10, 64}}, {T_LOWER, T_UPPER}});
     }
-    // the sweep schedule: level launches or the persistent single-block form
-    // (not tried when the levels average more than 16 passes of the block:
-    // one block cannot keep up with a full-width level launch there)
+    // the sweep schedule: level launches or the chained form (not tried when
+    // the levels average more than 4,096 cells: one cluster cannot keep up
+    // with a full-width level launch there)
     const int nlev = std::max<int>(1, int(c->lowOff.size()) - 1);
-    if (c->nCells / nlev <= 16 * kSeqThreads)
+    if (c->nCells / nlev <= 4096) {
+        if ((rc = build_chain(c))) return rc;
         groups.push_back({&T.sweep_persistent, nullptr, {{0, 0}, {1, 0}}, {T_LOWER, T_UPPER}});
+    }
     for (Cand &g : groups) {
         const int a0 = *g.a, b0 = g.b ? *g.b : 0;
         double best = 1e30, first = 0.0;
@@ -1667,6 +1784,7 @@ int ofg_autotune(ofg_ctx *c, int reps, ofg_tuning *out) {
     cudaEventDestroy(e1);
     T.ms_default = msDefault;
     T.ms_tuned = msTuned;
+    c->tuneSet = true;
     destroy_graphs(c);
     {
         std::lock_guard<std::mutex> g(g_tuneMutex);

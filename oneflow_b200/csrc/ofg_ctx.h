@@ -9,6 +9,15 @@
 #include "../../include/oneflow_b200.h"
 #include "ofg_device.cuh"
 
+namespace ofg {
+// One chained sweep's schedule on the device (ofg_chain.cuh)
+struct ChainBuf {
+    int *lev = nullptr, *ref = nullptr, *edge = nullptr, *cell = nullptr;
+    int nlev = 0, far = 0;
+    long long slots = 0;
+};
+}  // namespace ofg
+
 struct ofg_ctx {
     ofg_params p{};
     ofg::DevParams dp{};
@@ -33,7 +42,11 @@ struct ofg_ctx {
     int *d_nb_off = nullptr, *d_nbl = nullptr;              // per-cell neighbour lists (int2 pairs)
     int *d_lo_off = nullptr, *d_lol = nullptr, *d_up_off = nullptr, *d_upl = nullptr;
     int *d_lowOrder = nullptr, *d_upOrder = nullptr, *d_key = nullptr;
-    int *d_lowOff = nullptr, *d_upOff = nullptr;           // level offsets of the sweeps (persistent form)
+    ofg::ChainBuf chain[2];                                 // lower, upper (built when the chained sweeps are in use)
+    void *d_chainCoef = nullptr;                            // edge coefficients of the sweep under way
+    double *d_chainCell = nullptr;                          // and its cells' values, in the sweep's order
+    unsigned *chainStatus = nullptr;                        // pinned: a chained sweep's wait ran out
+    bool tuneSet = false;                                   // launch shapes chosen by the caller or the autotuner
     void *d_fgeo = nullptr, *d_cgeo = nullptr;              // face / cell records at the face precision
     double *d_fgeoD = nullptr;                              // mixed path: FP64 face records
     float *d_fofs = nullptr;                                // mixed path: face-local offsets [F][FOFS]

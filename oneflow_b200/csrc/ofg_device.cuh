@@ -42,7 +42,14 @@ template <> struct MinBlocks<float> {
 };
 
 constexpr int kRedBlocks = 148;   // blocks of the grid reductions (one per SM)
-constexpr int kSeqThreads = 512;  // threads of the one block of a persistent (single-block) sweep
+
+// chained sweeps (ofg_chain.cuh): warps of a level and groups of them in a block; ring positions
+constexpr int kChainWarps = 6, kChainGroups = 2, kChainThreads = 32 * kChainWarps * kChainGroups;
+constexpr int kChainRing = 4096, kChainMaxBlocks = 16;
+constexpr int kChainLevel = 16384;       // cells of a level: 64 bytes each stay below an mbarrier's 2^20 - 1
+constexpr int kChainNone = INT32_MIN;   // an empty edge slot
+constexpr int kEdgeCoefs = 15;          // values of an edge that do not depend on the increments
+constexpr int kChainCell = NEQ + 2;     // values of a cell: right-hand side, diagonal, its reciprocal
 
 constexpr int GLR = 24;   // gradient+limiter record: [var*3+dir] for 6 vars (q, T), limiter at 18..22
 constexpr int FGR = 8;    // face record: nx ny nz area xfc yfc zfc dist (|n . (x_r - x_l)|)

@@ -221,13 +221,48 @@ __global__ void __launch_bounds__(256) k_timestep_clip(KArgs<R> A) {
     A.rad[c] = s;
 }
 
-// x + (-y) / d without the division when it adds nothing: y = +0.0 and d > 0
-// give -0.0, and v + (-0.0) == v bit for bit.  (Measured: without the test,
-// the first upper-sweep level, whose cells have no later neighbours and so
-// y = +0.0, executed three times the instructions of the first lower level.)
-__device__ __forceinline__ double add_neg_quot(double x, double y, double d) {
-    if (y == 0.0 && !signbit(y) && d > 0.0) return x;
-    return x + (-y) / d;
+// y / d for the quotients of a sweep, one divisor for all five equations: r is
+// 1 / d, correctly rounded and formed ahead of the increments.  Two steps of
+// q += (y - d q) r end in the correctly rounded quotient (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34, 1990, theorem on q' = q + r (y - d q) for a faithful q)
+// while neither the remainder nor the quotient leaves the normal range, so
+// the result is y / d bit for bit for d and y in the middle of the range.  A zero numerator needs no
+// division at all (a 2-D solve's third momentum equation is all zeros, and
+// the compiler's division of a zero takes its slow path).
+struct Divisor {
+    double d, r;
+};
+__device__ __forceinline__ Divisor make_divisor(double d) { return Divisor{d, 1.0 / d}; }
+__device__ __forceinline__ bool mid_range(double a) { return a > 0x1p-300 && a < 0x1p300; }
+static __device__ __noinline__ double plain_div(double y, double d) { return y / d; }
+template <int N>
+__device__ __forceinline__ void div_by(const double *y, const Divisor &v, double *q) {
+    bool plain = mid_range(fabs(v.d));
+#pragma unroll
+    for (int e = 0; e < N; ++e) {   // without a branch, the N of them side by side
+        const double a = fabs(y[e]);
+        double t = __dmul_rn(y[e], v.r);
+        t = __fma_rn(__fma_rn(-v.d, t, y[e]), v.r, t);
+        t = __fma_rn(__fma_rn(-v.d, t, y[e]), v.r, t);
+        q[e] = a == 0.0 && v.d > 0.0 ? y[e] : t;
+        plain = plain && (a == 0.0 || mid_range(a));
+    }
+    if (plain) return;
+#pragma unroll
+    for (int e = 0; e < N; ++e) q[e] = plain_div(y[e], v.d);
+}
+
+// x + (-y) / d, where y = +0.0 and d > 0 leave x as it is, bit for bit
+// (-0.0 is added)
+template <int N>
+__device__ __forceinline__ void add_neg_quot(double *x, const double *y, const Divisor &v) {
+    double n[N], q[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e) n[e] = -y[e];
+    div_by<N>(n, v, q);
+#pragma unroll
+    for (int e = 0; e < N; ++e) x[e] += q[e];
 }
 
 // ---------------------------------------------------------------------------
@@ -1129,12 +1164,19 @@ __global__ void __launch_bounds__(128) k_face_sum(KArgs<float> A) {
 // and the viscous radius (UNsLusgs::CalcViscousTerm :295-330).  Level-scheduled:
 // every cell of a level only reads increments of cells in earlier levels.
 // ---------------------------------------------------------------------------
+// The increment's coefficients that do not depend on dq: the neighbour's split
+// eigenvalues and state, the face, the viscous radius.  Formed inside the
+// sweep by the level launches, ahead of it by the chained sweep.
+template <typename R> struct EdgeCoef {
+    R lmd1, x1, x2, c2, vn, af, htot, u, v, w, xn, yn, zn, fa, visrad;
+};
+
 // qa: the cell being solved (left after GCom::SetGeometry's swap), qb: neighbour;
 // dist = |n . (x_b - x_a)| (the face record's eighth slot, the same from both
 // sides), volb the neighbour's volume (read only for visSRModel 1)
 template <typename R>
-__device__ __forceinline__ void face_increment(const DevParams &P, const R *qa, const R *qb, const R *dqj, R xn,
-                                               R yn, R zn, R fa, R dist, R volb, double *rhs0) {
+__device__ __forceinline__ void edge_coef(const DevParams &P, const R *qa, const R *qb, R xn, R yn, R zn, R fa, R dist,
+                                          R volb, EdgeCoef<R> &E) {
     R vfn = R(0);
     R half = R(0.5), one = R(1), gl = R(P.gama), gr = gl;
     R rl = qa[IR], ul = qa[IU], vl = qa[IV], wl = qa[IW], pl = qa[IP];
@@ -1154,7 +1196,6 @@ __device__ __forceinline__ void face_increment(const DevParams &P, const R *qa, 
     R cmf = Rsqrt(c2f_);
     R vnf = xn * um + yn * vm + zn * wm;
     R maxEig = Rabs(vnf - vfn) + cmf;
-    R d0 = R(dqj[0]), d1 = R(dqj[1]), d2 = R(dqj[2]), d3 = R(dqj[3]), d4 = R(dqj[4]);
     R rj = rr, uj = ur, vj = vr, wj = wr, pj = pr;
     R c2 = Rabs(gama * pj / rj);
     R cm = Rsqrt(c2);
@@ -1164,51 +1205,76 @@ __device__ __forceinline__ void face_increment(const DevParams &P, const R *qa, 
     lmd1 = half * (lmd1 + (-maxEig));
     lmd2 = half * (lmd2 + (-maxEig));
     lmd3 = half * (lmd3 + (-maxEig));
-    R x1 = (lmd1 + lmd1 - lmd2 - lmd3) / (c2 + c2);
-    R x2 = (lmd2 - lmd3) / (cm + cm);
-    R dc = vn_fluid * d0 - xn * d1 - yn * d2 - zn * d3;
-    R c2dc = c2 * dc;
+    E.lmd1 = lmd1;
+    E.x1 = (lmd1 + lmd1 - lmd2 - lmd3) / (c2 + c2);
+    E.x2 = (lmd2 - lmd3) / (cm + cm);
+    E.c2 = c2;
+    E.vn = vn_fluid;
     R v2 = SQR3(uj, vj, wj);
-    R ae = gama - one, af = half * ae * v2;
-    R dh = -ae * (uj * d1 + vj * d2 + wj * d3 - d4);
+    R ae = gama - one;
+    E.af = half * ae * v2;
     R enthalpy = (gama / (gama - one)) * (pj / rj);
-    dh += af * d0;
-    R htot = enthalpy + half * v2;
-    R term1 = dh * x1 + dc * x2;
-    R term2 = c2dc * x1 + dh * x2;
-    R df[NEQ];
-    df[0] = lmd1 * d0 - term1;
-    df[1] = lmd1 * d1 - uj * term1 + xn * term2;
-    df[2] = lmd1 * d2 - vj * term1 + yn * term2;
-    df[3] = lmd1 * d3 - wj * term1 + zn * term2;
-    df[4] = lmd1 * d4 - htot * term1 + vn_fluid * term2;
-#pragma unroll
-    for (int e = 0; e < NEQ; ++e) df[e] *= fa;
+    E.htot = enthalpy + half * v2;
+    E.u = uj; E.v = vj; E.w = wj;
+    E.xn = xn; E.yn = yn; E.zn = zn; E.fa = fa;
+    E.visrad = R(0);
     if (P.vismodel > 0) {
         R vl_ = qb[IML], vt_ = qb[IMT];
-        R visrad;
         R density = half * (rl + rr);
         if (P.visSRModel == 1) {
             R c1 = R(4.0) / R(3.0) * (vl_ + vt_);
             R cc2 = R(P.gama) * (vl_ * R(P.oprl) + vt_ * R(P.oprt));
             R c3 = R(2) * Rmax(c1, cc2) / (R(P.reynolds) * density);
-            visrad = fa * fa * c3 / volb;
+            E.visrad = fa * fa * c3 / volb;
         } else {
             R viscosity = vl_ + vt_;
             R c1 = R(2) * viscosity / (density * dist * R(P.reynolds) + small_v<R>());
-            visrad = half * c1 * fa;
+            E.visrad = half * c1 * fa;
         }
-        rhs0[0] -= double(visrad * d0); rhs0[1] -= double(visrad * d1); rhs0[2] -= double(visrad * d2);
-        rhs0[3] -= double(visrad * d3); rhs0[4] -= double(visrad * d4);
+    }
+}
+
+// a b + c d: FP64 rounds both products, FP32 the first one alone (written
+// out, so that every kernel that uses it rounds alike)
+__device__ __forceinline__ double sum2(double a, double b, double c, double d) { return a * b + c * d; }
+__device__ __forceinline__ float sum2(float a, float b, float c, float d) { return __fmaf_rn(c, d, __fmul_rn(a, b)); }
+
+// The neighbour's increment dqj through the coefficients, added to rhs0
+template <typename R>
+__device__ __forceinline__ void edge_apply(const DevParams &P, const EdgeCoef<R> &E, const R *dqj, double *rhs0) {
+    R d0 = R(dqj[0]), d1 = R(dqj[1]), d2 = R(dqj[2]), d3 = R(dqj[3]), d4 = R(dqj[4]);
+    R dc = E.vn * d0 - E.xn * d1 - E.yn * d2 - E.zn * d3;
+    R c2dc = E.c2 * dc;
+    R ae = R(P.gama) - R(1);
+    R dh = -ae * (E.u * d1 + E.v * d2 + E.w * d3 - d4);
+    dh += E.af * d0;
+    R term1 = sum2(dh, E.x1, dc, E.x2);
+    R term2 = sum2(c2dc, E.x1, dh, E.x2);
+    R df[NEQ];
+    df[0] = E.lmd1 * d0 - term1;
+    df[1] = E.lmd1 * d1 - E.u * term1 + E.xn * term2;
+    df[2] = E.lmd1 * d2 - E.v * term1 + E.yn * term2;
+    df[3] = E.lmd1 * d3 - E.w * term1 + E.zn * term2;
+    df[4] = E.lmd1 * d4 - E.htot * term1 + E.vn * term2;
+#pragma unroll
+    for (int e = 0; e < NEQ; ++e) df[e] *= E.fa;
+    if (P.vismodel > 0) {
+        rhs0[0] -= double(E.visrad * d0); rhs0[1] -= double(E.visrad * d1); rhs0[2] -= double(E.visrad * d2);
+        rhs0[3] -= double(E.visrad * d3); rhs0[4] -= double(E.visrad * d4);
     }
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) rhs0[e] += double(df[e]);
 }
 
-// COH: the neighbours' increments are read with coherent loads, for a kernel
-// that itself wrote them earlier (the persistent sweep); otherwise through the
-// read-only path
-template <typename R, bool COH = false>
+template <typename R>
+__device__ __forceinline__ void face_increment(const DevParams &P, const R *qa, const R *qb, const R *dqj, R xn,
+                                               R yn, R zn, R fa, R dist, R volb, double *rhs0) {
+    EdgeCoef<R> E;
+    edge_coef(P, qa, qb, xn, yn, zn, fa, dist, volb, E);
+    edge_apply(P, E, dqj, rhs0);
+}
+
+template <typename R>
 __device__ __forceinline__ void sweep_rhs0(const KArgs<R> &A, int c, const int *off, const int2 *list, double *rhs0) {
     R qc[REC];
     ld8(A.qs + (size_t)c * REC, qc);
@@ -1221,10 +1287,7 @@ __device__ __forceinline__ void sweep_rhs0(const KArgs<R> &A, int c, const int *
         R qn[REC], fg[FGR], dqj[DQR];
         ld8(A.qs + (size_t)nb * REC, qn);
         ld8(A.fgeo + (size_t)f * FGR, fg);
-        // the neighbour's increment was written by an earlier level (an earlier
-        // launch, or an earlier pass of the persistent sweep)
-        if constexpr (COH) ldp8(A.dq + (size_t)nb * DQR, dqj);
-        else ld8(A.dq + (size_t)nb * DQR, dqj);
+        ld8(A.dq + (size_t)nb * DQR, dqj);   // written by an earlier level (an earlier launch)
         R volb = A.P.visSRModel == 1 ? A.cgeo[(size_t)nb * CGR + 3] : R(1);
         R xn = fg[0], yn = fg[1], zn = fg[2];
         if (nb_right(e2)) { xn = -xn; yn = -yn; zn = -zn; }   // GCom::SetGeometry
@@ -1232,29 +1295,37 @@ __device__ __forceinline__ void sweep_rhs0(const KArgs<R> &A, int c, const int *
     }
 }
 
-template <typename R, bool COH>
+template <typename R>
 __device__ __forceinline__ void lusgs_lower_cell(const KArgs<R> &A, int c) {
     double rhs0[NEQ] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    sweep_rhs0<R, COH>(A, c, A.lo_off, A.lol, rhs0);
-    double rad = A.rad[c];
+    sweep_rhs0(A, c, A.lo_off, A.lol, rhs0);
+    const Divisor rad = make_divisor(A.rad[c]);
     const double *rs = A.res + (size_t)c * NEQ;
+    double y[NEQ], v[NEQ];
+#pragma unroll
+    for (int e = 0; e < NEQ; ++e) y[e] = rs[e] - rhs0[e];
+    div_by<NEQ>(y, rad, v);
     R o[DQR];
 #pragma unroll
-    for (int e = 0; e < NEQ; ++e) o[e] = R((rs[e] - rhs0[e]) / rad);
+    for (int e = 0; e < NEQ; ++e) o[e] = R(v[e]);
     o[5] = o[6] = o[7] = R(0);
     st4(A.dq + (size_t)c * DQR, o);
     st4(A.dq + (size_t)c * DQR + 4, o + 4);
 }
 
-template <typename R, bool COH>
+template <typename R>
 __device__ __forceinline__ void lusgs_upper_cell(const KArgs<R> &A, int c) {
     double rhs0[NEQ] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    sweep_rhs0<R, COH>(A, c, A.up_off, A.upl, rhs0);   // ghost increments are zero: boundary faces not listed
-    double rad = A.rad[c];
+    sweep_rhs0(A, c, A.up_off, A.upl, rhs0);   // ghost increments are zero: boundary faces not listed
+    const Divisor rad = make_divisor(A.rad[c]);
     R o[DQR];
     ldp8(A.dq + (size_t)c * DQR, o);   // its own lower-sweep increment, rewritten below
+    double v[NEQ];
 #pragma unroll
-    for (int e = 0; e < NEQ; ++e) o[e] = R(add_neg_quot(double(o[e]), rhs0[e], rad));
+    for (int e = 0; e < NEQ; ++e) v[e] = double(o[e]);
+    add_neg_quot<NEQ>(v, rhs0, rad);
+#pragma unroll
+    for (int e = 0; e < NEQ; ++e) o[e] = R(v[e]);
     st4(A.dq + (size_t)c * DQR, o);
     st4(A.dq + (size_t)c * DQR + 4, o + 4);
 }
@@ -1263,40 +1334,13 @@ __device__ __forceinline__ void lusgs_upper_cell(const KArgs<R> &A, int c) {
 template <typename R, int MINB = MinBlocks<R>::sw>
 __global__ void __launch_bounds__(128, MINB) k_lusgs_lower(KArgs<R> A, const int *order, int start, int count) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < count) lusgs_lower_cell<R, false>(A, order[start + t]);
+    if (t < count) lusgs_lower_cell(A, order[start + t]);
 }
 
 template <typename R, int MINB = MinBlocks<R>::sw>
 __global__ void __launch_bounds__(128, MINB) k_lusgs_upper(KArgs<R> A, const int *order, int start, int count) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < count) lusgs_upper_cell<R, false>(A, order[start + t]);
-}
-
-// The persistent form: one block of kSeqThreads runs every level of the sweep
-// in order, with a block barrier between levels (a barrier also orders the
-// block's global writes before its later reads, so each level sees the
-// increments of the levels before it).  The same per-cell arithmetic as the
-// level launches, so the same bits; it replaces nlev launches by one, which
-// pays off when the levels are many and small (natural-order sweeps of
-// structured-like meshes: hundreds of levels of tens to hundreds of cells).
-template <typename R>
-__global__ void __launch_bounds__(kSeqThreads, 1) k_lusgs_lower_seq(KArgs<R> A, const int *order, const int *loff,
-                                                                 int nlev) {
-    for (int l = 0; l < nlev; ++l) {
-        const int st = loff[l], en = loff[l + 1];
-        for (int k = st + threadIdx.x; k < en; k += blockDim.x) lusgs_lower_cell<R, true>(A, order[k]);
-        __syncthreads();
-    }
-}
-
-template <typename R>
-__global__ void __launch_bounds__(kSeqThreads, 1) k_lusgs_upper_seq(KArgs<R> A, const int *order, const int *loff,
-                                                                 int nlev) {
-    for (int l = 0; l < nlev; ++l) {
-        const int st = loff[l], en = loff[l + 1];
-        for (int k = st + threadIdx.x; k < en; k += blockDim.x) lusgs_upper_cell<R, true>(A, order[k]);
-        __syncthreads();
-    }
+    if (t < count) lusgs_upper_cell(A, order[start + t]);
 }
 
 // ---------------------------------------------------------------------------

@@ -2,7 +2,10 @@
 // Included by one translation unit per precision (ofg_k64.cu is compiled
 // without FMA contraction so that the FP64 path rounds like the reference).
 #pragma once
+#include <algorithm>
+
 #include "ofg_ctx.h"
+#include "ofg_chain.cuh"
 #include "ofg_kernels.cuh"
 #include "ofg_turb.cuh"
 
@@ -130,6 +133,71 @@ void launch_flux(ofg_ctx *c, const KArgs<R> &A, cudaStream_t s, int part = 3) {
     }
 }
 
+// Blocks of a chained sweep's cluster, by the mean cells of a level.  A block
+// takes 32 kChainWarps = 192 cells of a level at once, two cells a thread
+// pipe-bound; a cluster pays about 0.4 us a level for its signals.  Measured,
+// us a sweep: 119 levels of 29 cells (FP64) 83 with one block, 107 with 4;
+// 385 of 170 (FP64) 565, 434, 450 with 1, 4, 8 blocks; 228 of 631 (FP64) 2,790,
+// 1,330, 1,120, 1,210 with 1, 4, 8, 16.
+inline int chain_blocks(const ofg_ctx *c) {
+    const int mean = c->nCells / std::max(1, c->chain[0].nlev);
+    return mean <= 96 ? 1 : mean <= 400 ? 4 : 8;
+}
+
+// Whether this context's sweeps run chained (one launch per sweep)
+inline bool chained(const ofg_ctx *c) { return c->tune.sweep_persistent && c->chain[0].lev && c->chain[1].lev; }
+
+inline ChainPlan chain_plan(const ofg_ctx *c, bool lower) {
+    const ChainBuf &b = c->chain[lower ? 0 : 1];
+    return ChainPlan{reinterpret_cast<const int4 *>(b.lev), lower ? c->d_lowOrder : c->d_upOrder, b.ref,
+                     reinterpret_cast<const int2 *>(b.edge), b.cell, b.nlev, b.far, b.slots, c->chainStatus};
+}
+
+template <typename K, typename... Args>
+int launch_chain(ofg_ctx *c, K one, K many, size_t smem, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = chain_blocks(c);
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    K kern = at.val.clusterDim.x > 1 ? many : one;
+    cfg.gridDim = dim3(at.val.clusterDim.x);
+    cfg.blockDim = dim3(kChainThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e == cudaSuccess && at.val.clusterDim.x > 8)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, kern, args...);
+    if (e != cudaSuccess) return c->fail(OFG_E_CUDA, std::string("chained sweep: ") + cudaGetErrorString(e));
+    ++c->launches;
+    return OFG_OK;
+}
+
+template <typename R, bool LOWER>
+int launch_chain_ns(ofg_ctx *c, const KArgs<R> &A, cudaStream_t s) {
+    const ChainPlan P = chain_plan(c, LOWER);
+    R *coef = static_cast<R *>(c->d_chainCoef);
+    OFG_LAUNCH((k_chain_coef<R, LOWER>), nblk(std::max<long long>(P.slots, A.nCells), 128), 128, s, A, P, coef,
+               c->d_chainCell);
+    return launch_chain(c, k_chain_ns<R, LOWER, false>, k_chain_ns<R, LOWER, true>,
+                        kChainRing * ChainNs<R, LOWER, true>::kBytes, s, A, P, (const R *)coef,
+                        (const double *)c->d_chainCell);
+}
+
+template <typename R, bool LOWER>
+int launch_chain_sa(ofg_ctx *c, const KArgs<R> &A, cudaStream_t s) {
+    const ChainPlan P = chain_plan(c, LOWER);
+    double *mat = static_cast<double *>(c->d_chainCoef);
+    OFG_LAUNCH((k_chain_mat<R, LOWER>), nblk(std::max<long long>(P.slots, A.nCells), 128), 128, s, A, P, mat,
+               c->d_chainCell);
+    return launch_chain(c, k_chain_sa<R, LOWER, false>, k_chain_sa<R, LOWER, true>,
+                        kChainRing * ChainSa<R, LOWER, true>::kBytes, s, A, P, (const double *)mat,
+                        (const double *)c->d_chainCell);
+}
+
 template <typename R>
 int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
     const int N = c->nCells;
@@ -175,10 +243,7 @@ int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
     case T_LOWER: {
         KArgs<R> A = make_args<R>(c, false);
         int nl = int(c->lowOff.size()) - 1;
-        if (c->tune.sweep_persistent) {
-            OFG_LAUNCH(k_lusgs_lower_seq<R>, 1, kSeqThreads, s, A, (const int *)c->d_lowOrder, (const int *)c->d_lowOff, nl);
-            break;
-        }
+        if (chained(c)) return launch_chain_ns<R, true>(c, A, s);
         for (int l = 0; l < nl; ++l) {
             int st = c->lowOff[l], cnt = c->lowOff[l + 1] - st;
             const int *ord = (const int *)c->d_lowOrder;
@@ -201,11 +266,7 @@ int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
         // unchanged bit for bit (add_neg_quot), so that level is not launched
         KArgs<R> A = make_args<R>(c, false);
         int nl = int(c->upOff.size()) - 1;
-        if (c->tune.sweep_persistent) {
-            OFG_LAUNCH(k_lusgs_upper_seq<R>, 1, kSeqThreads, s, A, (const int *)c->d_upOrder, (const int *)c->d_upOff + 1,
-                       nl - 1);
-            break;
-        }
+        if (chained(c)) return launch_chain_ns<R, false>(c, A, s);
         for (int l = 1; l < nl; ++l) {
             int st = c->upOff[l], cnt = c->upOff[l + 1] - st;
             const int *ord = (const int *)c->d_upOrder;
@@ -284,10 +345,7 @@ int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
     case T_TURB_LOWER: {
         KArgs<R> A = make_args<R>(c, true);
         int nl = int(c->lowOff.size()) - 1;
-        if (c->tune.sweep_persistent) {
-            OFG_LAUNCH(k_turb_lower_seq<R>, 1, kSeqThreads, s, A, (const int *)c->d_lowOrder, (const int *)c->d_lowOff, nl);
-            break;
-        }
+        if (chained(c)) return launch_chain_sa<R, true>(c, A, s);
         for (int l = 0; l < nl; ++l) {
             int st = c->lowOff[l], cnt = c->lowOff[l + 1] - st;
             OFG_LAUNCH(k_turb_lower<R>, nblk(cnt, 128), 128, s, A, (const int *)c->d_lowOrder, st, cnt);
@@ -297,11 +355,7 @@ int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
     case T_TURB_UPPER: {   // level 0 skipped, as in T_UPPER
         KArgs<R> A = make_args<R>(c, true);
         int nl = int(c->upOff.size()) - 1;
-        if (c->tune.sweep_persistent) {
-            OFG_LAUNCH(k_turb_upper_seq<R>, 1, kSeqThreads, s, A, (const int *)c->d_upOrder, (const int *)c->d_upOff + 1,
-                       nl - 1);
-            break;
-        }
+        if (chained(c)) return launch_chain_sa<R, false>(c, A, s);
         for (int l = 1; l < nl; ++l) {
             int st = c->upOff[l], cnt = c->upOff[l + 1] - st;
             OFG_LAUNCH(k_turb_upper<R>, nblk(cnt, 128), 128, s, A, (const int *)c->d_upOrder, st, cnt);

@@ -478,7 +478,10 @@ __device__ __forceinline__ void turb_lower_cell(const KArgs<R> &A, int c) {
         int f = nb_face(e2);
         rhs0 += (nb_right(e2) ? A.matL[f] : A.matR[f]) * A.dnut[e2.y];
     }
-    A.dnut[c] = (A.resT[c] - rhs0) / A.impsrT[c];
+    const double y = A.resT[c] - rhs0;
+    double q;
+    div_by<1>(&y, make_divisor(A.impsrT[c]), &q);
+    A.dnut[c] = q;
 }
 
 template <typename R>
@@ -489,35 +492,15 @@ __device__ __forceinline__ void turb_upper_cell(const KArgs<R> &A, int c) {
         int f = nb_face(e2);
         rhs0 += (nb_right(e2) ? A.matL[f] : A.matR[f]) * A.dnut[e2.y];
     }
-    A.dnut[c] = add_neg_quot(A.dnut[c], rhs0, A.impsrT[c]);
+    double v = A.dnut[c];
+    add_neg_quot<1>(&v, &rhs0, make_divisor(A.impsrT[c]));
+    A.dnut[c] = v;
 }
 
 template <typename R>
 __global__ void __launch_bounds__(128) k_turb_lower(KArgs<R> A, const int *order, int start, int count) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < count) turb_lower_cell(A, order[start + t]);
-}
-
-// the persistent forms (one block, every level, a barrier between levels; the
-// increments are read with plain, coherent loads)
-template <typename R>
-__global__ void __launch_bounds__(kSeqThreads, 1) k_turb_lower_seq(KArgs<R> A, const int *order, const int *loff,
-                                                                int nlev) {
-    for (int l = 0; l < nlev; ++l) {
-        const int st = loff[l], en = loff[l + 1];
-        for (int k = st + threadIdx.x; k < en; k += blockDim.x) turb_lower_cell(A, order[k]);
-        __syncthreads();
-    }
-}
-
-template <typename R>
-__global__ void __launch_bounds__(kSeqThreads, 1) k_turb_upper_seq(KArgs<R> A, const int *order, const int *loff,
-                                                                int nlev) {
-    for (int l = 0; l < nlev; ++l) {
-        const int st = loff[l], en = loff[l + 1];
-        for (int k = st + threadIdx.x; k < en; k += blockDim.x) turb_upper_cell(A, order[k]);
-        __syncthreads();
-    }
 }
 
 // UPDATE_FLOWFIELD (TurbUpdate::CalcFlowField1Equ, crelax = 1) fused with the
