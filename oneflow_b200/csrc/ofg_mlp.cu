@@ -263,10 +263,13 @@ __global__ void __launch_bounds__(GT, 1) k_gemm(int M, int N, int K, int kchunk,
     }
 }
 
-__device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float z) {
-    return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
+// GELU and its derivative from f = erf(z / sqrt 2)
+__device__ __forceinline__ float gelu_of(float z, float f) { return 0.5f * z * (1.0f + f); }
+__device__ __forceinline__ float gelu_grad_of(float z, float f) {
+    return 0.5f * (1.0f + f) + z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
+__device__ __forceinline__ float gelu(float z) { return gelu_of(z, erff(z * 0.70710678118654752f)); }
+__device__ __forceinline__ float gelu_grad(float z) { return gelu_grad_of(z, erff(z * 0.70710678118654752f)); }
 
 // Z += bias; H = bf16(GELU(Z))
 __global__ void k_bias_gelu(int64_t total, int N, float *Z, const float *bias, bf16 *H) {
@@ -333,8 +336,8 @@ __global__ void k_reduce_parts(int64_t n, int parts, const float *part, float *o
 }
 
 // loss of one minibatch: the rows' squared errors summed in FP64 in a fixed
-// order (thread-strided, then a shared-memory tree), one block
-__global__ void k_batch_loss(int rows, double scale, const float *rowErr, float *loss) {
+// order (thread-strided, then a shared-memory tree), one block of 256
+__device__ __forceinline__ void batch_loss(int rows, double scale, const float *rowErr, float *loss) {
     __shared__ double s[256];
     double a = 0.0;
     for (int r = threadIdx.x; r < rows; r += blockDim.x) a += rowErr[r];
@@ -346,20 +349,32 @@ __global__ void k_batch_loss(int rows, double scale, const float *rowErr, float 
     }
     if (threadIdx.x == 0) *loss = float(s[0] * scale);
 }
+__global__ void k_batch_loss(int rows, double scale, const float *rowErr, float *loss) {
+    batch_loss(rows, scale, rowErr, loss);
+}
 
-// Adam on the FP32 master copy, BF16 working copy refreshed; padded entries
-// (mask 0) stay zero
-__global__ void k_adam(int64_t n, float *w, float *m, float *v, const float *g, const unsigned char *mask,
-                       bf16 *wb, float lr, float b1, float b2, float eps, float c1, float c2) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n || (mask && !mask[i])) return;
-    float gi = g[i];
+// Adam on entry i of the FP32 master copy; returns the new value
+__device__ __forceinline__ float adam_step(float *w, float *m, float *v, float gi, int64_t i, float lr, float b1, float b2,
+                                           float eps, float c1, float c2) {
     float mi = b1 * m[i] + (1.0f - b1) * gi;
     float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
     m[i] = mi; v[i] = vi;
     float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     w[i] = wi;
+    return wi;
+}
+// Adam, BF16 working copy refreshed; padded entries (mask 0) stay zero
+__global__ void k_adam(int64_t n, float *w, float *m, float *v, const float *g, const unsigned char *mask,
+                       bf16 *wb, float lr, float b1, float b2, float eps, float c1, float c2) {
+    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n || (mask && !mask[i])) return;
+    const float wi = adam_step(w, m, v, g[i], i, lr, b1, b2, eps, c1, c2);
     if (wb) wb[i] = __float2bfloat16(wi);
+}
+
+__global__ void k_round(int64_t n, const float *w, bf16 *wb) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) wb[i] = __float2bfloat16(w[i]);
 }
 
 // minibatch rows: row r of step s takes sample hash(seed, s, r) mod n
@@ -391,6 +406,8 @@ __global__ void k_unpack_rows(int rows, int64_t n, int64_t r0, int N, int nout, 
     for (int c = 0; c < nout; ++c) Y[(r0 + r) * nout + c] = Z[(size_t)r * N + c];
 }
 
+#include "ofg_mlp_fused.cuh"
+
 }  // namespace
 
 struct ofg_mlp {
@@ -408,6 +425,14 @@ struct ofg_mlp {
     std::vector<bf16 *> H;                           // inputs of each layer [rows x K_l]
     bf16 *dZ = nullptr, *dHb = nullptr;              // [rows x maxdim]
     float *dH = nullptr, *part = nullptr, *Tb = nullptr, *rowErr = nullptr;
+    // the fused passes (ofg_mlp_fused.cuh) instead of wb, Z, H, dZ, dHb, dH and Tb
+    bool fused = false;
+    int pairs = 0;                     // pairs of blocks the device holds at once (0: not asked yet)
+    MlpNet net{};
+    bf16 *wf = nullptr, *wk = nullptr;
+    int capTiles = 0, capParts = 0;
+    bf16 *Hf = nullptr, *dZf = nullptr;
+    float *Gf = nullptr;
     long long adamStep = 0;
     bool gemmReady[4] = {false, false, false, false};   // k_gemm forms whose shared memory limit is raised
     std::string err;
@@ -427,8 +452,9 @@ void free_work(ofg_mlp *m) {
     for (auto p : m->H) cudaFree(p);
     m->Z.clear(); m->H.clear();
     cudaFree(m->dZ); cudaFree(m->dHb); cudaFree(m->dH); cudaFree(m->part); cudaFree(m->Tb); cudaFree(m->rowErr);
-    m->dZ = m->dHb = nullptr; m->dH = m->part = m->Tb = m->rowErr = nullptr;
-    m->capRows = 0;
+    cudaFree(m->Hf); cudaFree(m->dZf); cudaFree(m->Gf);
+    m->dZ = m->dHb = m->Hf = m->dZf = nullptr; m->dH = m->part = m->Tb = m->rowErr = m->Gf = nullptr;
+    m->capRows = m->capTiles = 0;
 }
 
 int ensure_work(ofg_mlp *m, int rows) {
@@ -521,6 +547,97 @@ int backward(ofg_mlp *m, int rows) {
     return OFG_OK;
 }
 
+// ---- the fused passes ----
+// Which networks: every layer's half fits a block's buffers.  Measured on the
+// 22 -> 6 x 256 -> 4 network: prediction of 294,912 rows 4.97 ms layer by layer,
+// 0.79 ms fused; a training step of 8,192 rows 0.55 ms, 0.13 ms.
+bool fits_fused(const ofg_mlp *m) {
+    if (m->L > kMlpLayers || m->N[m->L - 1] > kMlpOut) return false;
+    for (int l = 0; l < m->L; ++l)
+        if (m->K[l] > kMlpWidth || (l + 1 < m->L && m->N[l] > kMlpWidth)) return false;
+    return true;
+}
+
+void init_net(ofg_mlp *m) {
+    MlpNet &P = m->net;
+    P.L = m->L; P.nin = m->nin; P.nout = m->nout;
+    long long h = 0, z = 0;   // elements per row of the layers before
+    for (int l = 0; l < m->L; ++l) {
+        P.K[l] = m->K[l]; P.N[l] = m->N[l];
+        P.woff[l] = int(m->woff[l]); P.boff[l] = int(m->boff[l]);
+        P.hoff[l] = h * TILE_ROWS; P.zoff[l] = z * TILE_ROWS;
+        h += m->K[l]; z += m->N[l];
+    }
+    P.wf = m->wf; P.wk = m->wk; P.b = m->b;
+}
+
+// the BF16 working copies of the FP32 master weights
+int refresh_working(ofg_mlp *m) {
+    if (m->fused) k_mlp_pack<<<blocks(m->nw, 256), 256>>>(m->net, int(m->nw), m->w, m->wf, m->wk);
+    else k_round<<<blocks(m->nw, 256), 256>>>(int64_t(m->nw), m->w, m->wb);
+    MCK(cudaGetLastError());
+    return OFG_OK;
+}
+
+int fused_ready(ofg_mlp *m) {
+    if (m->pairs > 0) return OFG_OK;
+    MCK(cudaFuncSetAttribute(k_mlp_pass<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PASS));
+    MCK(cudaFuncSetAttribute(k_mlp_pass<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_PASS));
+    MCK(cudaFuncSetAttribute(k_mlp_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DW));
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 2;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(FT + 32);
+    cfg.dynamicSmemBytes = SMEM_PASS;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    MCK(cudaOccupancyMaxActiveClusters(&n, k_mlp_pass<false>, &cfg));
+    m->pairs = std::max(1, n);
+    return OFG_OK;
+}
+
+// buffers of the training passes over `rows` rows
+int ensure_fused(ofg_mlp *m, int rows) {
+    int rc = fused_ready(m);
+    if (rc) return rc;
+    const int tiles = (rows + TILE_ROWS - 1) / TILE_ROWS;
+    if (tiles <= m->capTiles) return OFG_OK;
+    free_work(m);
+    size_t h = 0, z = 0;
+    for (int l = 0; l < m->L; ++l) { h += m->K[l]; z += m->N[l]; }
+    const size_t n = (size_t)tiles * TILE_ROWS;
+    MCK(cudaMalloc(&m->Hf, n * h * sizeof(bf16)));
+    MCK(cudaMalloc(&m->dZf, n * z * sizeof(bf16)));
+    MCK(cudaMalloc(&m->Gf, n * z * sizeof(float)));
+    MCK(cudaMalloc(&m->part, SPLITK * m->nw * sizeof(float)));
+    MCK(cudaMalloc(&m->rowErr, n * sizeof(float)));
+    m->capTiles = tiles;
+    return OFG_OK;
+}
+
+// forth, back and the weight-gradient parts of one batch (R.rows rows)
+int fused_gradients(ofg_mlp *m, const MlpRows &R, int &parts) {
+    MlpNet &P = m->net;
+    P.H = m->Hf; P.dZ = m->dZf; P.G = m->Gf; P.rowErr = m->rowErr; P.tiles = m->capTiles;
+    const int tiles = (R.rows + TILE_ROWS - 1) / TILE_ROWS;
+    k_mlp_pass<true><<<2 * tiles, FT + 32, SMEM_PASS>>>(P, R);
+    DwGrid D{};
+    D.rows = R.rows;
+    D.chunk = pad16((R.rows + SPLITK - 1) / SPLITK);
+    D.parts = parts = (R.rows + D.chunk - 1) / D.chunk;
+    for (int l = 0; l < m->L; ++l)
+        D.first[l + 1] = D.first[l] + D.parts * int(blocks(m->K[l], BM)) * int(blocks(m->N[l], BN));
+    D.bias[0] = D.first[m->L];
+    for (int l = 0; l < m->L; ++l) D.bias[l + 1] = D.bias[l] + m->N[l] / 8;
+    k_mlp_dw<<<D.bias[m->L], DT, SMEM_DW>>>(P, D, m->part, m->gb);
+    MCK(cudaGetLastError());
+    return OFG_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -552,19 +669,23 @@ int ofg_mlp_create(int n_in, int width, int depth, int n_out, uint64_t seed, ofg
             }
         for (int j = 0; j < m->nfo[l]; ++j) bm[m->boff[l] + j] = 1;
     }
-    std::vector<bf16> wb(m->nw);
-    for (size_t i = 0; i < m->nw; ++i) wb[i] = __float2bfloat16(w[i]);
+    m->fused = fits_fused(m);
     auto fail = [&](cudaError_t e) { ofg_mlp_destroy(m); return e == cudaErrorMemoryAllocation ? OFG_E_NOMEM : OFG_E_CUDA; };
     cudaError_t e;
     float **fp[] = {&m->w, &m->mw, &m->vw, &m->gw};
     for (float **p : fp) if ((e = cudaMalloc(p, m->nw * sizeof(float))) != cudaSuccess) return fail(e);
     float **bp[] = {&m->b, &m->mb, &m->vb, &m->gb};
     for (float **p : bp) if ((e = cudaMalloc(p, m->nb * sizeof(float))) != cudaSuccess) return fail(e);
-    if ((e = cudaMalloc(&m->wb, m->nw * sizeof(bf16))) != cudaSuccess) return fail(e);
+    if (m->fused) {
+        for (bf16 **p : {&m->wf, &m->wk}) if ((e = cudaMalloc(p, m->nw * sizeof(bf16))) != cudaSuccess) return fail(e);
+    } else if ((e = cudaMalloc(&m->wb, m->nw * sizeof(bf16))) != cudaSuccess) {
+        return fail(e);
+    }
     if ((e = cudaMalloc(&m->wmask, m->nw)) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&m->bmask, m->nb)) != cudaSuccess) return fail(e);
     cudaMemcpy(m->w, w.data(), m->nw * sizeof(float), cudaMemcpyHostToDevice);
-    cudaMemcpy(m->wb, wb.data(), m->nw * sizeof(bf16), cudaMemcpyHostToDevice);
+    if (m->fused) init_net(m);
+    if (refresh_working(m) != OFG_OK) return fail(cudaErrorUnknown);
     cudaMemcpy(m->b, b.data(), m->nb * sizeof(float), cudaMemcpyHostToDevice);
     cudaMemcpy(m->wmask, wm.data(), m->nw, cudaMemcpyHostToDevice);
     cudaMemcpy(m->bmask, bm.data(), m->nb, cudaMemcpyHostToDevice);
@@ -579,7 +700,7 @@ void ofg_mlp_destroy(ofg_mlp *m) {
     if (!m) return;
     cudaDeviceSynchronize();
     free_work(m);
-    for (void *p : {(void *)m->w, (void *)m->b, (void *)m->wb, (void *)m->mw, (void *)m->vw, (void *)m->mb,
+    for (void *p : {(void *)m->wf, (void *)m->wk, (void *)m->w, (void *)m->b, (void *)m->wb, (void *)m->mw, (void *)m->vw, (void *)m->mb,
                     (void *)m->vb, (void *)m->gw, (void *)m->gb, (void *)m->wmask, (void *)m->bmask})
         cudaFree(p);
     delete m;
@@ -618,10 +739,8 @@ int ofg_mlp_set_params(ofg_mlp *m, const float *in) {
             for (int j = 0; j < m->nfo[l]; ++j) w[m->woff[l] + (size_t)i * m->N[l] + j] = in[o++];
         for (int j = 0; j < m->nfo[l]; ++j) b[m->boff[l] + j] = in[o++];
     }
-    std::vector<bf16> wb(m->nw);
-    for (size_t i = 0; i < m->nw; ++i) wb[i] = __float2bfloat16(w[i]);
     MCK(cudaMemcpy(m->w, w.data(), m->nw * sizeof(float), cudaMemcpyHostToDevice));
-    MCK(cudaMemcpy(m->wb, wb.data(), m->nw * sizeof(bf16), cudaMemcpyHostToDevice));
+    if (int rc = refresh_working(m)) return rc;
     MCK(cudaMemcpy(m->b, b.data(), m->nb * sizeof(float), cudaMemcpyHostToDevice));
     for (float *p : {m->mw, m->vw}) MCK(cudaMemset(p, 0, m->nw * sizeof(float)));
     for (float *p : {m->mb, m->vb}) MCK(cudaMemset(p, 0, m->nb * sizeof(float)));
@@ -632,6 +751,21 @@ int ofg_mlp_set_params(ofg_mlp *m, const float *in) {
 // Y[n][n_out] = f(X[n][n_in]) (device arrays, FP32), in blocks of `rows`
 int ofg_mlp_predict(ofg_mlp *m, const float *x, int64_t n, float *y) {
     if (!m || !x || !y || n < 0) return OFG_E_ARG;
+    if (m->fused) {
+        int rc = fused_ready(m);
+        if (rc) return rc;
+        const int64_t most = int64_t(1) << 30;   // rows of one launch (a multiple of the tile)
+        for (int64_t r0 = 0; r0 < n; r0 += most) {
+            MlpRows R{};
+            R.x = x + r0 * m->nin; R.out = y + r0 * m->nout;
+            R.rows = int(std::min(most, n - r0)); R.n = R.rows;
+            const int tiles = (R.rows + TILE_ROWS - 1) / TILE_ROWS;
+            k_mlp_pass<false><<<2 * std::min(tiles, m->pairs), FT + 32, SMEM_PASS>>>(m->net, R);
+        }
+        MCK(cudaGetLastError());
+        MCK(cudaDeviceSynchronize());
+        return gemm_status(m);
+    }
     const int rows = 16384;
     int rc = ensure_work(m, rows);
     if (rc) return rc;
@@ -652,11 +786,21 @@ int ofg_mlp_predict(ofg_mlp *m, const float *x, int64_t n, float *y) {
 int ofg_mlp_loss_grad(ofg_mlp *m, const float *x, const float *y, int64_t n, float *loss, float *grad) {
     if (!m || !x || !y || n <= 0 || n % ROWS || n > 65536) return OFG_E_ARG;
     int rows = int(n);
-    int rc = ensure_work(m, rows);
-    if (rc) return rc;
-    k_pack_rows<<<blocks(rows, 128), 128>>>(rows, n, 0, m->nin, m->K[0], x, m->H[0]);
-    MCK(cudaMemcpy(m->Tb, y, (size_t)rows * m->nout * sizeof(float), cudaMemcpyDeviceToDevice));
-    if ((rc = forward(m, rows, true)) || (rc = backward(m, rows))) return rc;
+    int rc;
+    if (m->fused) {
+        if ((rc = ensure_fused(m, rows))) return rc;
+        MlpRows R{};
+        R.x = x; R.y = y; R.n = n; R.rows = rows;
+        int parts = 0;
+        if ((rc = fused_gradients(m, R, parts))) return rc;
+        k_mlp_update<<<blocks(m->nw / 4, 256), 256>>>(m->net, int(m->nw), int(m->nb), parts, m->part, m->gw, m->gb, AdamStep{});
+        MCK(cudaGetLastError());
+    } else {
+        if ((rc = ensure_work(m, rows))) return rc;
+        k_pack_rows<<<blocks(rows, 128), 128>>>(rows, n, 0, m->nin, m->K[0], x, m->H[0]);
+        MCK(cudaMemcpy(m->Tb, y, (size_t)rows * m->nout * sizeof(float), cudaMemcpyDeviceToDevice));
+        if ((rc = forward(m, rows, true)) || (rc = backward(m, rows))) return rc;
+    }
     std::vector<float> e(rows), gw(m->nw), gb(m->nb);
     MCK(cudaMemcpy(e.data(), m->rowErr, rows * sizeof(float), cudaMemcpyDeviceToHost));
     MCK(cudaMemcpy(gw.data(), m->gw, m->nw * sizeof(float), cudaMemcpyDeviceToHost));
@@ -682,14 +826,30 @@ int ofg_mlp_loss_grad(ofg_mlp *m, const float *x, const float *y, int64_t n, flo
 int ofg_mlp_train(ofg_mlp *m, const float *x, const float *y, int64_t n, int batch, int steps, float lr,
                   uint64_t seed, float *loss_out) {
     if (!m || !x || !y || n <= 0 || batch <= 0 || batch % ROWS || batch > 65536 || steps < 0) return OFG_E_ARG;
-    int rc = ensure_work(m, batch);
+    int rc = m->fused ? ensure_fused(m, batch) : ensure_work(m, batch);
     if (rc) return rc;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     // the minibatch losses stay on the device until the end: no host
     // synchronisation between steps
     float *dLoss = nullptr;
     if (loss_out && steps > 0) MCK(cudaMalloc(&dLoss, (size_t)steps * sizeof(float)));
-    for (int s = 0; s < steps; ++s) {
+    for (int s = 0; s < steps && m->fused; ++s) {
+        MlpRows R{};
+        R.x = x; R.y = y; R.n = n; R.rows = batch;
+        R.hashed = true; R.seed = seed; R.step = uint64_t(s);
+        int parts = 0;
+        if ((rc = fused_gradients(m, R, parts))) {
+            cudaFree(dLoss);
+            return rc;
+        }
+        ++m->adamStep;
+        const float c1 = 1.0f - std::pow(b1, float(m->adamStep)), c2 = 1.0f - std::pow(b2, float(m->adamStep));
+        const AdamStep S{lr, b1, b2, eps, c1, c2, m->w, m->mw, m->vw, m->b, m->mb, m->vb, m->wf, m->wk, m->wmask,
+                         m->bmask, dLoss ? dLoss + s : nullptr, 1.0 / (double(batch) * m->nout), batch};
+        k_mlp_update<<<blocks(m->nw / 4, 256) + blocks(m->nb, 256) + (dLoss ? 1 : 0), 256>>>(
+            m->net, int(m->nw), int(m->nb), parts, m->part, nullptr, m->gb, S);
+    }
+    for (int s = 0; s < steps && !m->fused; ++s) {
         k_gather<<<blocks(batch, 128), 128>>>(batch, n, m->nin, m->K[0], m->nout, x, y, seed, uint64_t(s), m->H[0],
                                               m->Tb);
         if ((rc = forward(m, batch, true)) || (rc = backward(m, batch))) {
