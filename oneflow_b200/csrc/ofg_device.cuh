@@ -83,6 +83,50 @@ template <typename R> __device__ __forceinline__ R Rmax(R a, R b) { return a > b
 template <typename R> __device__ __forceinline__ R Rmin(R a, R b) { return a < b ? a : b; }
 template <typename R> __device__ __forceinline__ R SQR3(R a, R b, R c) { return a * a + b * b + c * c; }
 
+// y / d for the quotients of a sweep, one divisor for all five equations: r is
+// 1 / d, correctly rounded and formed ahead of the increments.  Two steps of
+// q += (y - d q) r end in the correctly rounded quotient (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34, 1990, theorem on q' = q + r (y - d q) for a faithful q)
+// while neither the remainder nor the quotient leaves the normal range, so
+// the result is y / d bit for bit for d and y in the middle of the range.  A zero numerator needs no
+// division at all (a 2-D solve's third momentum equation is all zeros, and
+// the compiler's division of a zero takes its slow path).
+struct Divisor {
+    double d, r;
+};
+__device__ __forceinline__ Divisor make_divisor(double d) { return Divisor{d, 1.0 / d}; }
+__device__ __forceinline__ bool mid_range(double a) { return a > 0x1p-300 && a < 0x1p300; }
+static __device__ __noinline__ double plain_div(double y, double d) { return y / d; }
+template <int N>
+__device__ __forceinline__ void div_by(const double *y, const Divisor &v, double *q) {
+    bool plain = mid_range(fabs(v.d));
+#pragma unroll
+    for (int e = 0; e < N; ++e) {   // without a branch, the N of them side by side
+        const double a = fabs(y[e]);
+        double t = __dmul_rn(y[e], v.r);
+        t = __fma_rn(__fma_rn(-v.d, t, y[e]), v.r, t);
+        t = __fma_rn(__fma_rn(-v.d, t, y[e]), v.r, t);
+        q[e] = a == 0.0 && v.d > 0.0 ? y[e] : t;
+        plain = plain && (a == 0.0 || mid_range(a));
+    }
+    if (plain) return;
+#pragma unroll
+    for (int e = 0; e < N; ++e) q[e] = plain_div(y[e], v.d);
+}
+
+// x + (-y) / d, where y = +0.0 and d > 0 leave x as it is, bit for bit
+// (-0.0 is added)
+template <int N>
+__device__ __forceinline__ void add_neg_quot(double *x, const double *y, const Divisor &v) {
+    double n[N], q[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e) n[e] = -y[e];
+    div_by<N>(n, v, q);
+#pragma unroll
+    for (int e = 0; e < N; ++e) x[e] += q[e];
+}
+
 // Constant parameters of one solve (reference script keys + derived state,
 // codes/chemical/src/Chemical.cpp:280-340, codes/ns/src/NsCom.cpp:45-94).
 struct DevParams {

@@ -22,18 +22,22 @@
 // the same update formulas; only its inner products are summed in a
 // different (blocked, deterministic) order.
 //
-// GMRES on the device: per Krylov step two kernels.  k_gm_spmv_dots scales
-// the previous unnormalised vector on read, stores the new basis vector,
-// forms w = A v and, per 256-row chunk, the chunk's share of every inner
-// product V[r] . w (one warp per r), summed per block in shared memory; the
-// last block to finish (ticket counter, no waiting) sums the blocks' shares
-// into column j of the Hessenberg matrix.  k_gm_orth subtracts the projections row by row in the reference's
-// order and sums |w|^2; its last block applies the earlier rotations and the
-// new one to column j, updates the rotated residual and decides convergence.
-// The host launches the steps in chunks and reads one flag per chunk; a step
-// launched after convergence returns at once.
+// GMRES on the device: per Krylov step three kernels, without a ticket or a
+// last block between them.  k_gm_spmv_dots sums the previous step's |w|^2 for
+// itself, scales the previous unnormalised vector on read, stores the new basis
+// vector, forms w = A v and, per 256-row chunk, the chunk's share of every inner
+// product V[r] . w (one warp per r; the products are split over several blocks
+// a chunk, so that a small system fills the chip too); one block more applies
+// the Givens rotations of the previous step's column, updates the rotated
+// residual and decides convergence.  k_gm_hsum adds the chunks' shares of the
+// new Hessenberg column.  k_gm_orth subtracts the projections row by row in the
+// reference's order and leaves |w|^2 by warps.  Every sum keeps one fixed
+// order whatever the grid.  The host launches the steps in chunks and reads one
+// flag per chunk; a step launched after convergence returns at once.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -50,6 +54,11 @@ constexpr double kTol = 1.0e-8;      // its tolerance
 constexpr int kThreads = 256;
 constexpr int kChunk = kThreads;     // rows per block of k_gm_spmv_dots (one per thread)
 constexpr int kStepsPerSync = 8;     // Krylov steps launched between flag reads
+constexpr int kHCol = kKrylov + 1;   // entries of a Hessenberg column
+constexpr int kOrth = 128;           // rows of a k_gm_orth block: half of a 256-row block
+constexpr int kOrthVec = 32, kOrthRing = 2;   // vectors of a stage, stages
+constexpr int kOrthBox = 16;         // vectors of one copy
+constexpr int kDotsSmem = (kThreads / 32) * 4 * kChunk * 8, kOrthSmem = kOrthRing * kOrthVec * kOrth * 8;
 
 // face record [nFaces][kFR]
 enum : int {
@@ -61,12 +70,12 @@ __device__ __forceinline__ double max0(double v) { return 0.0 > v ? 0.0 : v; }  
 
 // GMRES scalars shared by the kernels of one solve
 struct GmState {
-    int j;          // current Krylov step
     int done;       // 1 once converged or out of steps
     int dim;        // dimension of the update (the step that converged, or kKrylov - 1)
     int iters;      // steps counted as the reference returns them
     double normRHS, rho, inv, res;
     unsigned int ticket;
+    int timeout;    // a bounded wait ran out
 };
 
 struct Dev {
@@ -442,12 +451,15 @@ struct Gm {
     const double *A;
     const double *b;   // right-hand side
     double *x;         // solution
-    double *V;         // [kKrylov + 1][nT] normalised basis
+    double *V;         // [kKrylov + 1][ld] normalised basis (ld: nT in whole 128 bytes, for the bulk copies)
+    size_t ld;
     double *W;         // [nT] unnormalised next vector
     double *Y;         // [nT] A v_j
-    double *H;         // [(kKrylov + 1) * kKrylov] row-major (i, j) -> i * kKrylov + j
+    double *H;         // [kKrylov][kHCol]: column after column
     double *gc, *gs, *s;
-    double *part;      // [nBlk][kKrylov + 1] per-chunk inner products, then [nBlk] norms
+    double *part;      // [kKrylov + 1][nChunkBlk] shares of the inner products
+    double *wpart;     // [nGrid][kThreads / 32] shares of |w|^2, by warps of 256-row blocks
+    int nChunkBlk, nGrid;
     GmState *st;
 };
 
@@ -502,7 +514,6 @@ __global__ void k_gm_init(Gm G) {
     S->res = normr1;
     if (normRHS < 1.0e-5) normRHS = 1.0;
     S->normRHS = normRHS;
-    S->j = 0;
     S->iters = 0;
     S->dim = -1;
     S->ticket = 0;
@@ -512,36 +523,201 @@ __global__ void k_gm_init(Gm G) {
     S->inv = 1.0 / normr1;
 }
 
-// one Krylov step, first half: v_j = W / |W| (stored), Y = A v_j, and the
-// inner products V[r] . Y, r <= j, into column j of H.  Each block walks its
-// 256-row chunks (grid stride), forms the chunk's rows of A v_j in shared
-// memory and adds the chunk's share of each product to its own sum in shared
-// memory (warp r % 8 owns r); its sums go out r-major, and the last block
-// (ticket counter, no waiting) adds the blocks' sums for each r with a warp
-// over the blocks -- a fixed order throughout.
-__global__ void __launch_bounds__(kThreads) k_gm_spmv_dots(Gm G) {
+// ---- tiles of the basis into shared memory by TMA, counted on an mbarrier ----
+constexpr unsigned kWaitLimit = 1u << 20;   // try_wait rounds before a wait gives up
+__device__ __forceinline__ uint32_t gm_smem(const void *p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void gm_bar_init(uint32_t bar, uint32_t n) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(n) : "memory");
+}
+__device__ __forceinline__ void gm_bar_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+__device__ __forceinline__ void gm_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void gm_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// rows [x, x + box) of basis vectors [y, y + box): one copy (x a multiple of the box, so 16-byte aligned)
+__device__ __forceinline__ void gm_tile(uint32_t dst, const CUtensorMap &map, int x, int y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(&map), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ bool gm_wait(uint32_t bar, uint32_t parity) {
+    for (unsigned i = 0; i < kWaitLimit; ++i) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+// A Krylov step's kernels are launched before the one ahead of them ends: each
+// lets the next one's blocks in as soon as its own run, and reads what the
+// one ahead wrote after gm_ahead (measured at the launches)
+__device__ __forceinline__ void gm_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void gm_ahead() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// |w| of the last k_gm_orth, by a whole block of kThreads: the warps' shares of
+// each 256-row block, the blocks over the threads (strided), the block's tree
+__device__ __forceinline__ double gm_norm(const Gm &G, double *sh) {
+    __shared__ double norm;
+    double v = 0.0;
+    for (int b = threadIdx.x; b < G.nGrid; b += kThreads) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; ++w) t += __ldcg(G.wpart + (size_t)b * (kThreads / 32) + w);
+        v += t;
+    }
+    const double sum = block_sum(v, sh);
+    if (threadIdx.x == 0) norm = sqrt(sum);
+    __syncthreads();
+    return norm;
+}
+
+// The Givens rotations of column `col` (H holds it as the products left it,
+// normr2 = |w| goes below the diagonal), the rotated residual and the decision
+__device__ void gm_givens(const Gm &G, int col, double normr2) {
+    __shared__ double run[kHCol], rc[kKrylov], rs[kKrylov], pc[kKrylov], ps[kKrylov];
+    double *h = G.H + (size_t)col * kHCol;
+    // row's rotation of (hr, h(row + 1)) gives h(row) = c hr + s h(row + 1) and
+    // the next hr = -s hr + c h(row + 1): only the running entry hr is serial,
+    // the products with h(row + 1) and the results are not
+    for (int r = threadIdx.x; r < col; r += blockDim.x) {
+        const double c = G.gc[r], sn = G.gs[r], hn = h[r + 1];
+        rc[r] = c; rs[r] = sn; pc[r] = c * hn; ps[r] = sn * hn;
+    }
+    if (threadIdx.x == 0) run[0] = h[0];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double hr = run[0];
+        int row = 0;
+        for (; row + 8 <= col; row += 8) {
+            double sn[8], p[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) { sn[q] = rs[row + q]; p[q] = pc[row + q]; }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                hr = -sn[q] * hr + p[q];
+                run[row + q + 1] = hr;
+            }
+        }
+        for (; row < col; ++row) {
+            hr = -rs[row] * hr + pc[row];
+            run[row + 1] = hr;
+        }
+        GmState *S = G.st;
+        double hcc = hr, hc1 = normr2, c, sn;   // h(col, col), h(col + 1, col)
+        if (hc1 == 0.0) {
+            c = 1.0; sn = 0.0;
+        } else if (fabs(hc1) > fabs(hcc)) {
+            double tmp = hcc / hc1;
+            sn = 1.0 / sqrt(1.0 + tmp * tmp);
+            c = tmp * sn;
+        } else {
+            double tmp = hc1 / hcc;
+            c = 1.0 / sqrt(1.0 + tmp * tmp);
+            sn = tmp * c;
+        }
+        G.gc[col] = c; G.gs[col] = sn;
+        {
+            double tmp = c * hcc + sn * hc1;
+            hc1 = -sn * hcc + c * hc1;
+            hcc = tmp;
+        }
+        if (hc1 < 1e-10) hc1 = 0;
+        h[col] = hcc;
+        h[col + 1] = hc1;
+        const double s0 = G.s[col], s1 = G.s[col + 1];
+        const double st = c * s0 + sn * s1, Sv = -sn * s0 + c * s1;
+        G.s[col + 1] = Sv;
+        G.s[col] = st;
+        S->rho = sqrt(Sv * Sv);
+        if (S->rho < kTol * S->normRHS) {
+            S->dim = col; S->iters = col; S->done = 1;
+        } else if (col + 1 == kKrylov) {
+            S->dim = kKrylov - 1; S->iters = kKrylov; S->done = 1;
+        }
+    }
+    __syncthreads();
+    for (int r = threadIdx.x; r < col; r += blockDim.x) h[r] = rc[r] * run[r] + ps[r];
+}
+
+// One Krylov step, first part: v_j = W / |W| (stored), Y = A v_j, and the
+// shares of the inner products V[r] . Y, r <= j.  Blocks (b, g): b walks its
+// 256-row chunks (grid stride over nChunkBlk), forms the chunk's rows of A v_j in
+// shared memory and adds the chunk's share of each product to its own sum
+// (a warp owns four r a pass; g takes every gridDim.y-th round of passes).
+// Block (nChunkBlk, 0) finishes the column before.  Measured, us on average over
+// a 500-step solve of 16,900 rows: 11.0 with loads of 32 values a lane, 8.6 with
+// tiles by TMA (the rotations beside them: 17 us for 500 rows with the column
+// rotated in place, 7 with only its running entry serial); 65,800 rows 35.6, 25.1.
+// What bounds it: its start (4 us: |w|, a root, a quotient, a row of A), then
+// L2 / HBM.
+__global__ void __launch_bounds__(kThreads, 3) k_gm_spmv_dots(Gm G, int j, const __grid_constant__ CUtensorMap tiles) {
+    extern __shared__ __align__(128) double ring[];   // [warp][4][kChunk]
     __shared__ double ys[kChunk];
     __shared__ double acc[kKrylov + 1];
-    __shared__ bool last;
+    __shared__ double sh[32];
+    __shared__ uint64_t bars[kThreads / 32];
+    const int nT = G.nT;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = kThreads / 32;
+    const int g = blockIdx.y, G4 = 4 * nw * gridDim.y;
+    const uint32_t bar = gm_smem(bars + wid), mine = gm_smem(ring + (size_t)wid * 4 * kChunk);
+    uint32_t phase = 0;
+    gm_next();
+    if (lane == 0) {
+        gm_bar_init(bar, 1);
+        gm_bar_fence();
+    }
+    __syncwarp();
+    gm_ahead();
     GmState *S = G.st;
     if (((volatile int *)&S->done)[0]) return;
-    const int j = S->j;
-    const double inv = S->inv;
-    const int nT = G.nT;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    double *Vj = G.V + (size_t)j * nT;
+    double inv = 0.0;
+    if (j > 0) {
+        const double norm = gm_norm(G, sh);
+        if (blockIdx.x == G.nChunkBlk) {
+            if (g == 0) gm_givens(G, j - 1, norm);
+            return;
+        }
+        inv = 1.0 / norm;
+    } else {
+        if (blockIdx.x == G.nChunkBlk) return;
+        inv = S->inv;
+    }
+    if (g > 0 && 4 * nw * g >= j) return;
+    double *Vj = G.V + (size_t)j * G.ld;
     for (int r = threadIdx.x; r <= j; r += blockDim.x) acc[r] = 0.0;
     const int nChunks = (nT + kChunk - 1) / kChunk;
-    for (int ch = blockIdx.x; ch < nChunks; ch += gridDim.x) {
+    for (int ch = blockIdx.x; ch < nChunks; ch += G.nChunkBlk) {
         const int r0 = ch * kChunk;
+        // a pass's 8 KB come by one copy; the first one's ahead of the rows of A
+        auto copy = [&](int rb) {
+            if (rb >= j || lane != 0) return;
+            gm_expect(bar, 4 * kChunk * 8);
+            gm_tile(mine, tiles, r0, rb, bar);
+        };
+        const int first = 4 * (wid + nw * g);
+        copy(first);
         __syncthreads();   // ys of the previous chunk consumed
         {
             const int t = threadIdx.x, i = r0 + t;
             double y = 0.0;
             if (i < nT) {
-                Vj[i] = G.W[i] * inv;
                 for (int k = G.rOff[i]; k < G.rOff[i + 1]; ++k) y += G.A[k] * (G.W[G.JA[k]] * inv);
-                G.Y[i] = y;
+                if (g == 0) {
+                    Vj[i] = G.W[i] * inv;
+                    G.Y[i] = y;
+                }
             }
             ys[t] = y;
         }
@@ -552,207 +728,236 @@ __global__ void __launch_bounds__(kThreads) k_gm_spmv_dots(Gm G) {
         double yv[KR];
 #pragma unroll
         for (int k = 0; k < KR; ++k) yv[k] = ys[lane + 32 * k];
-        // v_j = W * inv for the lane's rows (this step's vector, not stored yet)
-        double wv[KR];
+        // the stored basis vectors r < j, four per pass of the warp, each summed
+        // over the lane's rows in ascending order, then over the warp; a pass's
+        // 8 KB come by bulk copies, the next pass's while this one's are summed
+        const double *ring0 = ring + (size_t)wid * 4 * kChunk;
+        for (int rb = first; rb < j; rb += G4) {
+            const bool ok = gm_wait(bar, phase);
+            phase ^= 1;
+            if (!__all_sync(0xffffffffu, ok)) {
+                S->timeout = 1;
+                gm_wait(bar, phase ^ 1);   // the copy in flight, once more
+                break;
+            }
+            double v[4][KR];
 #pragma unroll
-        for (int k = 0; k < KR; ++k) wv[k] = lane + 32 * k < rows ? G.W[r0 + lane + 32 * k] * inv : 0.0;
-        // the stored basis vectors r < j, four per pass of the warp (32 loads
-        // in flight per lane), each summed over the lane's rows in ascending
-        // order, then over the warp; warp w owns r with (r / 4) % 8 == w
-        for (int rb = 4 * wid; rb < j; rb += 4 * nw) {
-            const double *V0 = G.V + (size_t)rb * nT + r0;
-            double d0 = 0.0, d1 = 0.0, d2 = 0.0, d3 = 0.0;
-            if (rows == kChunk && rb + 4 <= j) {   // the common case: no guards
-                double a[KR], b[KR], c[KR], e[KR];
+            for (int q = 0; q < 4; ++q)
 #pragma unroll
-                for (int k = 0; k < KR; ++k) {
-                    const int t = lane + 32 * k;
-                    a[k] = __ldg(V0 + t);
-                    b[k] = __ldg(V0 + nT + t);
-                    c[k] = __ldg(V0 + 2 * (size_t)nT + t);
-                    e[k] = __ldg(V0 + 3 * (size_t)nT + t);
-                }
+                for (int k = 0; k < KR; ++k) v[q][k] = ring0[q * kChunk + lane + 32 * k];
+            __syncwarp();
+            copy(rb + G4);
+            double d[4] = {0.0, 0.0, 0.0, 0.0};
+            if (rows == kChunk) {
 #pragma unroll
-                for (int k = 0; k < KR; ++k) {
-                    d0 += yv[k] * a[k]; d1 += yv[k] * b[k]; d2 += yv[k] * c[k]; d3 += yv[k] * e[k];
-                }
+                for (int k = 0; k < KR; ++k)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) d[q] += yv[k] * v[q][k];
             } else {
 #pragma unroll
-                for (int k = 0; k < KR; ++k) {
-                    const int t = lane + 32 * k;
-                    if (t < rows) {
-                        d0 += yv[k] * __ldg(V0 + t);
-                        if (rb + 1 < j) d1 += yv[k] * __ldg(V0 + nT + t);
-                        if (rb + 2 < j) d2 += yv[k] * __ldg(V0 + 2 * (size_t)nT + t);
-                        if (rb + 3 < j) d3 += yv[k] * __ldg(V0 + 3 * (size_t)nT + t);
+                for (int k = 0; k < KR; ++k)
+                    if (lane + 32 * k < rows) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) d[q] += yv[k] * v[q][k];
                     }
-                }
             }
             for (int o = 16; o > 0; o >>= 1) {
-                d0 += __shfl_down_sync(0xffffffffu, d0, o);
-                d1 += __shfl_down_sync(0xffffffffu, d1, o);
-                d2 += __shfl_down_sync(0xffffffffu, d2, o);
-                d3 += __shfl_down_sync(0xffffffffu, d3, o);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) d[q] += __shfl_down_sync(0xffffffffu, d[q], o);
             }
             if (lane == 0) {
-                acc[rb] += d0;
-                if (rb + 1 < j) acc[rb + 1] += d1;
-                if (rb + 2 < j) acc[rb + 2] += d2;
-                if (rb + 3 < j) acc[rb + 3] += d3;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (rb + q < j) acc[rb + q] += d[q];
             }
         }
-        // r = j, by the warp that owns it
-        if (((j / 4) % nw) == wid) {
+        // r = j: this step's vector, not stored yet
+        if (g == 0 && wid == nw - 1) {
             double d = 0.0;
 #pragma unroll
             for (int k = 0; k < KR; ++k)
-                if (lane + 32 * k < rows) d += yv[k] * wv[k];
+                if (lane + 32 * k < rows) d += yv[k] * (G.W[r0 + lane + 32 * k] * inv);
             for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
             if (lane == 0) acc[j] += d;
         }
     }
     __syncthreads();
-    const int nb = gridDim.x;
-    for (int r = threadIdx.x; r <= j; r += blockDim.x) G.part[(size_t)r * nb + blockIdx.x] = acc[r];
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(&S->ticket, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    // column j of H: per r, the lanes over the blocks' sums (fixed order) and
-    // a warp reduction; a warp takes four r per pass (four loads in flight)
-    for (int rq = 4 * wid; rq <= j; rq += 4 * nw) {
-        double h[4] = {0.0, 0.0, 0.0, 0.0};
-        const double *P = G.part + (size_t)rq * nb;
-        for (int b = lane; b < nb; b += 32) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (rq + q <= j) h[q] += __ldcg(P + (size_t)q * nb + b);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            for (int o = 16; o > 0; o >>= 1) h[q] += __shfl_down_sync(0xffffffffu, h[q], o);
-            if (lane == 0 && rq + q <= j) G.H[(size_t)(rq + q) * kKrylov + j] = h[q];
-        }
-    }
-    if (threadIdx.x == 0) S->ticket = 0;
+    // this block's products: rounds of 4 nw of them, every gridDim.y-th one
+    for (int r = threadIdx.x; r <= j; r += blockDim.x)
+        if (r == j ? g == 0 : r % G4 / (4 * nw) == g) G.part[(size_t)r * G.nChunkBlk + blockIdx.x] = acc[r];
 }
 
-// one Krylov step, second half: W = Y - sum_r V[r] H[r][j] (subtracted in
-// order r = 0..j, as the reference), |W|^2, then (last block) H[j+1][j],
-// the Givens rotations of column j, the rotated residual and the decision
-__global__ void __launch_bounds__(kThreads) k_gm_orth(Gm G) {
-    __shared__ double sh[32];
-    __shared__ double hcol[kKrylov + 1];
-    __shared__ double rc[kKrylov], rs[kKrylov];   // the last block's copy of the earlier rotations
-    __shared__ bool last;
+// Column j of H: per r, a warp's lanes over the blocks' shares (strided), then
+// the warp's tree
+__global__ void __launch_bounds__(kThreads) k_gm_hsum(Gm G, int j) {
+    gm_next();
+    gm_ahead();
+    if (((volatile int *)&G.st->done)[0]) return;
+    const int lane = threadIdx.x & 31, r = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    if (r > j) return;
+    const double *P = G.part + (size_t)r * G.nChunkBlk;
+    double h = 0.0;
+#pragma unroll 4
+    for (int b = lane; b < G.nChunkBlk; b += 32) h += __ldcg(P + b);
+    for (int o = 16; o > 0; o >>= 1) h += __shfl_down_sync(0xffffffffu, h, o);
+    if (lane == 0) G.H[(size_t)j * kHCol + r] = h;
+}
+
+// One Krylov step, second part: W = Y - sum_r V[r] H[r][j] (subtracted in
+// order r = 0..j, as the reference), and |W|^2 by warps.  One warp copies the
+// basis vectors of the block's 128 rows ahead of the others, kOrthVec at a
+// time into a ring of kOrthRing.  Measured, us on average over a 500-step solve
+// of 16,900 / 65,800 rows: 13.7 / 34.8 with 32 loads a thread ahead; 14.7 / 30.9 with
+// a copy a vector (an SM takes some 75 cycles for each, however small) and
+// eight vectors a stage; 10.8 / 26.2 with 32; 6.4 / 23.2 with tiles of 16 vectors
+// by one TMA instruction, 0.87 of the measured HBM rate at the larger size.
+__global__ void __launch_bounds__(kOrth + 32, 3) k_gm_orth(Gm G, int j, const __grid_constant__ CUtensorMap tiles) {
+    extern __shared__ __align__(128) double ring[];   // [kOrthRing][kOrthVec][kOrth]
+    __shared__ double hcol[kHCol];
+    __shared__ uint64_t bars[2 * kOrthRing];          // full, then free
+    const int nT = G.nT, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t full = gm_smem(bars), free_ = full + 8 * kOrthRing;
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < kOrthRing; ++k) {
+            gm_bar_init(full + 8 * k, 1);
+            gm_bar_init(free_ + 8 * k, kOrth / 32);
+        }
+        gm_bar_fence();
+    }
+    gm_next();
+    gm_ahead();
     GmState *S = G.st;
     if (((volatile int *)&S->done)[0]) return;
-    const int j = S->j;
-    const int nT = G.nT;
-    for (int r = threadIdx.x; r <= j; r += blockDim.x) hcol[r] = G.H[(size_t)r * kKrylov + j];
+    for (int r = threadIdx.x; r <= j; r += blockDim.x) hcol[r] = __ldcg(G.H + (size_t)j * kHCol + r);
     __syncthreads();
-    double v = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nT; i += gridDim.x * blockDim.x) {
-        double w = G.Y[i];
-        // in the reference's order r = 0..j; the basis entries of 16 steps
-        // are loaded together ahead of their subtractions
-        int r = 0;
-        for (; r + 16 <= j + 1; r += 16) {
-            double vv[16];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) vv[q] = __ldg(G.V + (size_t)(r + q) * nT + i);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) w = w - vv[q] * hcol[r + q];
+    const int step = G.nGrid * kThreads, passes = (j + kOrthVec) / kOrthVec;
+    int n = 0;   // passes so far, over all rows
+    if (warp == kOrth / 32) {
+        bool ok = true;
+        for (int i0 = blockIdx.x * kOrth; i0 < nT && ok; i0 += step)
+            for (int p = 0; p < passes; ++p, ++n) {
+                const int k = n % kOrthRing, boxes = (min(kOrthVec, j + 1 - kOrthVec * p) + kOrthBox - 1) / kOrthBox;
+                if (n >= kOrthRing) ok = __all_sync(0xffffffffu, gm_wait(free_ + 8 * k, (n / kOrthRing - 1) & 1));
+                if (!ok) break;
+                if (lane == 0) {
+                    gm_expect(full + 8 * k, boxes * kOrthBox * kOrth * 8);
+                    for (int q = 0; q < boxes; ++q)
+                        gm_tile(gm_smem(ring + (size_t)(k * kOrthVec + q * kOrthBox) * kOrth), tiles, i0,
+                                kOrthVec * p + q * kOrthBox, full + 8 * k);
+                }
+            }
+        if (!ok) {
+            S->timeout = 1;
+            for (int q = max(0, n - kOrthRing); q < n; ++q)   // the copies in flight
+                gm_wait(full + 8 * (q % kOrthRing), (q / kOrthRing) & 1);
         }
-        for (; r <= j; ++r) w = w - __ldg(G.V + (size_t)r * nT + i) * hcol[r];
-        G.W[i] = w;
-        v += w * w;
+        return;
     }
-    double t = block_sum(v, sh);
-    if (threadIdx.x == 0) {
-        G.part[blockIdx.x] = t;
-        __threadfence();
-        last = atomicAdd(&S->ticket, 1u) == gridDim.x - 1;
+    double v = 0.0;
+    bool ok = true;
+    for (int i0 = blockIdx.x * kOrth; i0 < nT && ok; i0 += step) {
+        const int i = i0 + threadIdx.x;
+        double w = i < nT ? G.Y[i] : 0.0;
+        for (int p = 0; p < passes; ++p, ++n) {
+            const int k = n % kOrthRing, m = min(kOrthVec, j + 1 - kOrthVec * p);
+            ok = __all_sync(0xffffffffu, gm_wait(full + 8 * k, (n / kOrthRing) & 1));
+            if (!ok) {
+                S->timeout = 1;
+                break;
+            }
+            const double *u = ring + (size_t)k * kOrthVec * kOrth + threadIdx.x;
+            if (m == kOrthVec) {
+                double vv[kOrthVec];
+#pragma unroll
+                for (int q = 0; q < kOrthVec; ++q) vv[q] = u[q * kOrth];
+                __syncwarp();
+                if (lane == 0) gm_arrive(free_ + 8 * k);
+#pragma unroll
+                for (int q = 0; q < kOrthVec; ++q) w = w - vv[q] * hcol[kOrthVec * p + q];
+            } else {
+                for (int q = 0; q < m; ++q) w = w - u[q * kOrth] * hcol[kOrthVec * p + q];
+                __syncwarp();
+                if (lane == 0) gm_arrive(free_ + 8 * k);
+            }
+        }
+        if (i < nT) {
+            G.W[i] = w;
+            v += w * w;
+        }
     }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    const double sum = last_block_sum(G.part, gridDim.x, 1, sh);
-    for (int r = threadIdx.x; r < j; r += blockDim.x) { rc[r] = G.gc[r]; rs[r] = G.gs[r]; }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    const double normr2 = sqrt(sum);
-    double *H = G.H;
-    auto h = [&](int a, int b) -> double & { return H[(size_t)a * kKrylov + b]; };
-    const int col = j;
-    // the earlier rotations down column j (hcol holds it as the products left
-    // it): the running entry h(row, col) stays in a register, the rotated
-    // entries go out as they are final
-    double hr = hcol[0];
-    for (int row = 0; row < col; ++row) {
-        const double hn = hcol[row + 1], c = rc[row], sn = rs[row];
-        double tmp = c * hr + sn * hn;
-        hr = -sn * hr + c * hn;
-        h(row, col) = tmp;
-    }
-    double hcc = hr, hc1 = normr2;   // h(col, col), h(col + 1, col)
-    if (hc1 == 0.0) {
-        G.gc[col] = 1.0; G.gs[col] = 0.0;
-    } else if (fabs(hc1) > fabs(hcc)) {
-        double tmp = hcc / hc1;
-        G.gs[col] = 1.0 / sqrt(1.0 + tmp * tmp);
-        G.gc[col] = tmp * G.gs[col];
-    } else {
-        double tmp = hc1 / hcc;
-        G.gc[col] = 1.0 / sqrt(1.0 + tmp * tmp);
-        G.gs[col] = tmp * G.gc[col];
-    }
-    {
-        const double c = G.gc[col], sn = G.gs[col];
-        double tmp = c * hcc + sn * hc1;
-        hc1 = -sn * hcc + c * hc1;
-        hcc = tmp;
-    }
-    if (hc1 < 1e-10) hc1 = 0;
-    h(col, col) = hcc;
-    h(col + 1, col) = hc1;
-    const double st = G.gc[col] * G.s[col] + G.gs[col] * G.s[col + 1];
-    G.s[col + 1] = -G.gs[col] * G.s[col] + G.gc[col] * G.s[col + 1];
-    G.s[col] = st;
-    const double Sv = G.s[j + 1];
-    S->rho = sqrt(Sv * Sv);
-    S->inv = 1.0 / normr2;
-    S->ticket = 0;
-    if (S->rho < kTol * S->normRHS) {
-        S->dim = j; S->iters = j; S->done = 1;
-    } else if (j + 1 == kKrylov) {
-        S->dim = kKrylov - 1; S->iters = kKrylov; S->done = 1;
-    } else {
-        S->j = j + 1;
-    }
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) G.wpart[(size_t)blockIdx.x * (kOrth / 32) + warp] = v;
 }
 
-// Update (GMRES.h:20-61), first part: back substitution of s in place
-__global__ void k_gm_backsub(Gm G) {
-    GmState *S = G.st;
-    const int dim = S->dim;
-    for (int l = dim; l >= 0; --l) {
-        if (threadIdx.x == 0) G.s[l] = G.s[l] / G.H[(size_t)l * kKrylov + l];
-        __syncthreads();
-        const double sl = G.s[l];
-        for (int i = threadIdx.x; i < l; i += blockDim.x) G.s[i] -= sl * G.H[(size_t)i * kKrylov + l];
-        __syncthreads();
-    }
+// the last column's rotations, after the last step
+__global__ void __launch_bounds__(kThreads) k_gm_finish(Gm G, int col) {
+    __shared__ double sh[32];
+    if (((volatile int *)&G.st->done)[0]) return;
+    gm_givens(G, col, gm_norm(G, sh));
 }
 
-// x += V s, basis vectors from the last (GMRES.h:47-60)
-__global__ void k_gm_update_x(Gm G) {
+// Update (GMRES.h:20-61), first part: back substitution of s in place (the
+// diagonal's reciprocals formed ahead of the serial chain)
+__global__ void __launch_bounds__(kThreads) k_gm_backsub(Gm G) {
+    __shared__ double s[kKrylov], d[kKrylov], rd[kKrylov], sl;
+    const int dim = G.st->dim;
+    for (int l = threadIdx.x; l <= dim; l += blockDim.x) {
+        s[l] = G.s[l];
+        d[l] = G.H[(size_t)l * kHCol + l];
+        rd[l] = 1.0 / d[l];
+    }
+    // this thread's entries of the next columns, loaded kAhead columns ahead
+    constexpr int kMine = (kKrylov + kThreads - 1) / kThreads, kAhead = 8;
+    double next[kAhead][kMine];
+    auto column = [&](int l, double *to) {
+#pragma unroll
+        for (int k = 0; k < kMine; ++k) {
+            const int i = threadIdx.x + k * kThreads;
+            to[k] = i < l ? G.H[(size_t)l * kHCol + i] : 0.0;   // (l < 0: none)
+        }
+    };
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) column(dim - q, next[q]);
+    __syncthreads();
+    for (int l0 = dim; l0 >= 0; l0 -= kAhead) {
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) {
+            const int l = l0 - q;
+            if (l < 0) break;
+            if (threadIdx.x == 0) {
+                double v;
+                ofg::div_by<1>(&s[l], ofg::Divisor{d[l], rd[l]}, &v);
+                s[l] = v;
+                sl = v;
+            }
+            __syncthreads();
+            const double t = sl;
+#pragma unroll
+            for (int k = 0; k < kMine; ++k) {
+                const int i = threadIdx.x + k * kThreads;
+                if (i < l) s[i] -= t * next[q][k];
+            }
+            column(l - kAhead, next[q]);
+            __syncthreads();
+        }
+    }
+    for (int l = threadIdx.x; l <= dim; l += blockDim.x) G.s[l] = s[l];
+}
+
+// x += V s, basis vectors from the last (GMRES.h:47-60), 16 loaded ahead
+__global__ void __launch_bounds__(kOrth) k_gm_update_x(Gm G) {
     const int dim = G.st->dim;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < G.nT; i += gridDim.x * blockDim.x) {
         double x = G.x[i];
-        for (int m = dim; m >= 0; --m) x += G.V[(size_t)m * G.nT + i] * G.s[m];
+        int m = dim;
+        for (; m >= 15; m -= 16) {
+            double vv[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) vv[q] = __ldg(G.V + (size_t)(m - q) * G.ld + i);
+#pragma unroll
+            for (int q = 0; q < 16; ++q) x += vv[q] * __ldg(G.s + m - q);
+        }
+        for (; m >= 0; --m) x += G.V[(size_t)m * G.ld + i] * G.s[m];
         G.x[i] = x;
     }
 }
@@ -792,11 +997,13 @@ struct ofg_ins {
     std::vector<void *> allocs;
     // GMRES workspace
     double *V = nullptr, *W = nullptr, *Y = nullptr, *H = nullptr, *gc = nullptr, *gs = nullptr, *s = nullptr,
-           *gpart = nullptr;
+           *gpart = nullptr, *wpart = nullptr;
     GmState *st = nullptr;
     GmState *hst = nullptr;           // pinned host copy of the GMRES scalars
     double *hred = nullptr;           // pinned host copy of remax
     int nPart = 0, nChunkBlk = 0, nGrid = 0;
+    size_t ld = 0;                    // between basis vectors
+    CUtensorMap dotTiles{}, orthTiles{};   // of the basis: 256 rows x 4 vectors, 128 x kOrthBox
     long long nnz = 0;
     long innerSteps = 0;
     double remax[4] = {1, 1, 1, 1};
@@ -825,33 +1032,79 @@ namespace {
 
 int blocks(int n) { return (n + kThreads - 1) / kThreads; }
 
+// The basis V [kKrylov + 1][ld] as tiles of `rows` rows x `vectors` vectors
+bool basis_tiles(const ofg_ins *s, int rows, int vectors, CUtensorMap *map) {
+    using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess || !fn) return false;
+    const cuuint64_t size[2] = {s->ld, kKrylov + 1}, stride[1] = {s->ld * sizeof(double)};
+    const cuuint32_t box[2] = {(cuuint32_t)rows, (cuuint32_t)vectors}, step[2] = {1, 1};
+    return reinterpret_cast<Encode>(fn)(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, s->V, size, stride, box, step,
+                                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// a launch whose blocks may, where `early`, start before the kernel ahead of it ends (it waits by gm_ahead)
+template <typename K, typename... Args>
+cudaError_t launch_early(bool early, K kern, dim3 grid, int block, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // one GMRES solve of A x = b on the context's stream; returns OFG_OK and the
 // iteration count / residual in *its, *res
 int gmres(ofg_ins *s, const double *A, const double *b, double *x, int *its, double *res) {
     cudaStream_t st = s->c->stream;
     Gm G{};
     G.nT = s->D.nT; G.rOff = s->D.rOff; G.JA = s->D.JA; G.A = A; G.b = b; G.x = x;
-    G.V = s->V; G.W = s->W; G.Y = s->Y; G.H = s->H; G.gc = s->gc; G.gs = s->gs; G.s = s->s; G.part = s->gpart;
+    G.V = s->V; G.ld = s->ld; G.W = s->W; G.Y = s->Y; G.H = s->H; G.gc = s->gc; G.gs = s->gs; G.s = s->s; G.part = s->gpart;
+    G.wpart = s->wpart; G.nChunkBlk = s->nChunkBlk; G.nGrid = s->nGrid;
     G.st = s->st;
     INS_CK(cudaEventRecord(s->eg0, st));
-    INS_CK(cudaMemsetAsync(s->H, 0, sizeof(double) * (size_t)(kKrylov + 1) * kKrylov, st));
     INS_CK(cudaMemsetAsync(s->s, 0, sizeof(double) * (kKrylov + 1), st));
     INS_CK(cudaMemsetAsync(&s->st->ticket, 0, sizeof(unsigned int), st));
     k_gm_init<<<s->nGrid, kThreads, 0, st>>>(G);
+    INS_CK(cudaFuncSetAttribute(k_gm_spmv_dots, cudaFuncAttributeMaxDynamicSharedMemorySize, kDotsSmem));
+    INS_CK(cudaFuncSetAttribute(k_gm_orth, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrthSmem));
+    // early launches pay while a kernel's start counts: us a Krylov step without
+    // and with them 22.8 / 16.8 (17 x 17), 26.2 / 24.6 (128 x 128), 61.8 / 60.2
+    // (256 x 256), 212.6 / 215.0 (512 x 512: the next kernel's blocks hold slots)
+    const bool early = s->D.nT < 100000;
+    // blocks a chunk: enough for two an SM
+    const int split = std::max(1, std::min(4, 296 / s->nChunkBlk));
     for (int step = 0; step < kKrylov;) {
         for (int k = 0; k < kStepsPerSync && step < kKrylov; ++k, ++step) {
-            k_gm_spmv_dots<<<s->nChunkBlk, kThreads, 0, st>>>(G);
-            k_gm_orth<<<s->nGrid, kThreads, 0, st>>>(G);
+            INS_CK(launch_early(early, k_gm_spmv_dots, dim3(s->nChunkBlk + 1, split), kThreads, kDotsSmem, st, G, step, s->dotTiles));
+            INS_CK(launch_early(early, k_gm_hsum, dim3((step + kThreads / 32) / (kThreads / 32)), kThreads, 0, st, G, step));
+            INS_CK(launch_early(early, k_gm_orth, dim3(s->nGrid * (kThreads / kOrth)), kOrth + 32, kOrthSmem, st, G, step,
+                                s->orthTiles));
         }
+        if (step == kKrylov) k_gm_finish<<<1, kThreads, 0, st>>>(G, kKrylov - 1);
         INS_CK(cudaGetLastError());
         INS_CK(cudaMemcpyAsync(s->hst, s->st, sizeof(GmState), cudaMemcpyDeviceToHost, st));
         INS_CK(cudaStreamSynchronize(st));
+        if (s->hst->timeout) {
+            INS_CK(cudaMemsetAsync(&s->st->timeout, 0, sizeof(int), st));
+            return s->fail(OFG_E_TIMEOUT, "a GMRES wait ran out");
+        }
         if (s->hst->done) break;
     }
     if (!s->hst->done) return s->fail(OFG_E_STATE, "GMRES did not finish");
     if (s->hst->dim >= 0) {
         k_gm_backsub<<<1, kThreads, 0, st>>>(G);
-        k_gm_update_x<<<s->nGrid, kThreads, 0, st>>>(G);
+        k_gm_update_x<<<s->nGrid * (kThreads / kOrth), kOrth, 0, st>>>(G);
         k_gm_residual<<<s->nGrid, kThreads, 0, st>>>(G);
         INS_CK(cudaGetLastError());
         INS_CK(cudaMemcpyAsync(s->hst, s->st, sizeof(GmState), cudaMemcpyDeviceToHost, st));
@@ -1029,15 +1282,17 @@ int ofg_ins_create(ofg_ctx *c, const double *wall_uvw, ofg_ins **out) {
     }
     s->nGrid = std::min(blocks(nT), 148 * 8);
     s->nPart = std::max(s->nChunkBlk * (kKrylov + 1), s->nGrid);
-    z(&s->V, (size_t)(kKrylov + 1) * T); z(&s->W, T); z(&s->Y, T);
+    s->ld = (T + 15) / 16 * 16;
+    z(&s->V, (size_t)(kKrylov + 1) * s->ld); z(&s->W, T); z(&s->Y, T);
     z(&s->H, (size_t)(kKrylov + 1) * kKrylov); z(&s->gc, kKrylov); z(&s->gs, kKrylov); z(&s->s, kKrylov + 1);
-    z(&s->gpart, (size_t)s->nPart);
+    z(&s->gpart, (size_t)s->nPart); z(&s->wpart, (size_t)s->nGrid * (kThreads / 32));
     if (!rc) rc = s->alloc(&s->st, 1);
     if (!rc && cudaMallocHost((void **)&s->hst, sizeof(GmState)) != cudaSuccess) rc = OFG_E_NOMEM;
     if (!rc && cudaMallocHost((void **)&s->hred, 4 * sizeof(double)) != cudaSuccess) rc = OFG_E_NOMEM;
     if (!rc && (cudaEventCreate(&s->ev0) != cudaSuccess || cudaEventCreate(&s->ev1) != cudaSuccess ||
                 cudaEventCreate(&s->eg0) != cudaSuccess || cudaEventCreate(&s->eg1) != cudaSuccess))
         rc = OFG_E_CUDA;
+    if (!rc && (!basis_tiles(s, kChunk, 4, &s->dotTiles) || !basis_tiles(s, kOrth, kOrthBox, &s->orthTiles))) rc = OFG_E_CUDA;
     s->nnz = rOff[nT];
     if (!rc && (cudaMemset(D.ticket, 0, sizeof(unsigned)) != cudaSuccess ||
                 cudaMemset(s->st, 0, sizeof(GmState)) != cudaSuccess ||
