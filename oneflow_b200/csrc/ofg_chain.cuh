@@ -365,8 +365,7 @@ struct ChainNs {
     }
     __device__ __forceinline__ void store() const {
         const R o[DQR] = {R(own[0]), R(own[1]), R(own[2]), R(own[3]), R(own[4]), R(0), R(0), R(0)};
-        st4(A.dq + (size_t)c * DQR, o);
-        st4(A.dq + (size_t)c * DQR + 4, o + 4);
+        st8(A.dq + (size_t)c * DQR, o);
     }
 };
 

@@ -54,30 +54,55 @@ __device__ __forceinline__ void ld4(const float *p, float *o) {
     float4 a = __ldg(reinterpret_cast<const float4 *>(p));
     o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
 }
+// 32 bytes at once (p 32-byte aligned: every record but the FP32 cell and
+// nu~-gradient records is whole 32-byte sectors).  These gathers wait on memory
+// with a quarter to half of the warps an SM holds; half as many requests for
+// the same bytes took, of 16-byte loads' time, the gradients 86 -> 78 us, the
+// face pass 82 -> 78, the lower sweep 77 -> 67, the upper 56 -> 44, the update 30 -> 24
+// (600,000 tetrahedra, mixed).
 __device__ __forceinline__ void ld4(const double *p, double *o) {
-    double2 a = __ldg(reinterpret_cast<const double2 *>(p)), b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
-    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3]) : "l"(p));
 }
-template <typename T> __device__ __forceinline__ void ld8(const T *p, T *o) { ld4(p, o); ld4(p + 4, o + 4); }
+__device__ __forceinline__ void ld8(const float *p, float *o) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
+        : "l"(p));
+}
+__device__ __forceinline__ void ld8(const double *p, double *o) { ld4(p, o); ld4(p + 4, o + 4); }
 // plain (coherent) vector loads, for a record the same launch writes afterwards
 __device__ __forceinline__ void ldp8(const float *p, float *o) {
-    float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
-    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
+                 : "l"(p)
+                 : "memory");
 }
 __device__ __forceinline__ void ldp8(const double *p, double *o) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        double2 a = reinterpret_cast<const double2 *>(p)[i];
-        o[2 * i] = a.x; o[2 * i + 1] = a.y;
-    }
+    for (int i = 0; i < 8; i += 4)
+        asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                     : "=d"(o[i]), "=d"(o[i + 1]), "=d"(o[i + 2]), "=d"(o[i + 3])
+                     : "l"(p + i)
+                     : "memory");
 }
 
 __device__ __forceinline__ void st4(float *p, const float *v) {
     *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
 __device__ __forceinline__ void st4(double *p, const double *v) {
-    reinterpret_cast<double2 *>(p)[0] = make_double2(v[0], v[1]);
-    reinterpret_cast<double2 *>(p)[1] = make_double2(v[2], v[3]);
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
+                 : "memory");
+}
+__device__ __forceinline__ void st8(float *p, const float *v) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void st8(double *p, const double *v) { st4(p, v); st4(p + 4, v + 4); }
+
+// a gradient+limiter record (GLR values)
+template <typename R> __device__ __forceinline__ void ld_gl(const R *p, R *o) {
+#pragma unroll
+    for (int i = 0; i < GLR; i += 8) ld8(p + i, o + i);
 }
 
 // Block reductions for 1-D blocks of up to 1024 threads (a multiple of 32),
@@ -467,7 +492,7 @@ __global__ void __launch_bounds__(128, MINB) k_gradlim(KArgs<R> A, int nvar, int
         rec[23] = R(0);
         R *o = A.gl + (size_t)c * GLR;
 #pragma unroll
-        for (int i = 0; i < GLR; i += 4) st4(o + i, rec + i);
+        for (int i = 0; i < GLR; i += 8) st8(o + i, rec + i);
         if (limMode == 2) {
             R *m = A.mm + (size_t)c * MMR;
 #pragma unroll
@@ -538,8 +563,7 @@ __global__ void __launch_bounds__(128) k_limiter_global(KArgs<R> A) {
     R cgc[CGR], rec[GLR];
     ld4(A.cgeo + (size_t)c * CGR, cgc);
     R *o = A.gl + (size_t)c * GLR;
-#pragma unroll
-    for (int i = 0; i < GLR; i += 4) ld4(o + i, rec + i);
+    ld_gl(o, rec);
     const R *m = A.mm + (size_t)c * MMR;
     R mn[NEQ], mx[NEQ], eps[NEQ], lim[NEQ];
 #pragma unroll
@@ -894,8 +918,7 @@ __global__ void __launch_bounds__(128, MinBlocks<R>::res) k_residual(KArgs<R> A)
         vol = double(cgc[3]);
         bool needGl = doRes && (P.ilim != -1 || P.vismodel > 0);
         if (needGl) {
-#pragma unroll
-            for (int i = 0; i < GLR; i += 4) ld4(A.gl + (size_t)c * GLR + i, glc + i);
+            ld_gl(A.gl + (size_t)c * GLR, glc);
         }
         R gam = R(P.gama), ce1 = R(P.centropy1), ce2 = R(P.centropy2), orey = R(P.oreynolds);
         int b = A.nb_off[c], en = A.nb_off[c + 1];
@@ -913,8 +936,7 @@ __global__ void __launch_bounds__(128, MinBlocks<R>::res) k_residual(KArgs<R> A)
             ld4(A.cgeo + (size_t)nb * CGR, cgn);
             bool ghost = nb >= A.nCells;
             if (needGl && !ghost) {
-#pragma unroll
-                for (int i = 0; i < GLR; i += 4) ld4(A.gl + (size_t)nb * GLR + i, gln + i);
+                ld_gl(A.gl + (size_t)nb * GLR, gln);
             }
             const R *ql = right ? qn : qc, *qr = right ? qc : qn;
             const R *cgl = right ? cgn : cgc, *cgr = right ? cgc : cgn;
@@ -949,8 +971,7 @@ __global__ void __launch_bounds__(128, MinBlocks<R>::res) k_residual(KArgs<R> A)
                 ld4(A.cgeo + (size_t)nb * CGR, cgn);
                 bool ghost = nb >= A.nCells;
                 if (!ghost) {
-#pragma unroll
-                    for (int i = 0; i < GLR; i += 4) ld4(A.gl + (size_t)nb * GLR + i, gln + i);
+                    ld_gl(A.gl + (size_t)nb * GLR, gln);
                 }
                 const R *ql = right ? qn : qc, *qr = right ? qc : qn;
                 const R *cgl = right ? cgn : cgc, *cgr = right ? cgc : cgn;
@@ -1029,15 +1050,13 @@ __global__ void __launch_bounds__(128, MINB) k_face_pass(KArgs<float> A) {
     if (doRes) {
         float gll[GLR], glr[GLR];
         if (P.ilim != -1 || P.vismodel > 0) {
-#pragma unroll
-            for (int i = 0; i < GLR; i += 4) ld4(A.gl + (size_t)lr.x * GLR + i, gll + i);
+            ld_gl(A.gl + (size_t)lr.x * GLR, gll);
             // a ghost cell carries its interior cell's gradient (UGrad.cpp:140-148)
             if (bface) {
 #pragma unroll
                 for (int i = 0; i < GLR; ++i) glr[i] = gll[i];
             } else {
-#pragma unroll
-                for (int i = 0; i < GLR; i += 4) ld4(A.gl + (size_t)lr.y * GLR + i, glr + i);
+                ld_gl(A.gl + (size_t)lr.y * GLR, glr);
             }
         }
         const float gam = float(P.gama), ce1 = float(P.centropy1), ce2 = float(P.centropy2);
@@ -1265,8 +1284,7 @@ __device__ __forceinline__ void lusgs_lower_cell(const KArgs<R> &A, int c) {
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) o[e] = R(v[e]);
     o[5] = o[6] = o[7] = R(0);
-    st4(A.dq + (size_t)c * DQR, o);
-    st4(A.dq + (size_t)c * DQR + 4, o + 4);
+    st8(A.dq + (size_t)c * DQR, o);
 }
 
 template <typename R>
@@ -1282,8 +1300,7 @@ __device__ __forceinline__ void lusgs_upper_cell(const KArgs<R> &A, int c) {
     add_neg_quot<NEQ>(v, rhs0, rad);
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) o[e] = R(v[e]);
-    st4(A.dq + (size_t)c * DQR, o);
-    st4(A.dq + (size_t)c * DQR + 4, o + 4);
+    st8(A.dq + (size_t)c * DQR, o);
 }
 
 // one level of a sweep per launch (cells order[start .. start+count))
@@ -1326,8 +1343,7 @@ __global__ void __launch_bounds__(128) k_calc_lhs(KArgs<R> A, double coef) {
         }
 #pragma unroll
         for (int e = NEQ; e < DQR; ++e) d[e] = R(0);
-        st4(A.dq + (size_t)c * DQR, d);
-        st4(A.dq + (size_t)c * DQR + 4, d + 4);
+        st8(A.dq + (size_t)c * DQR, d);
     }
     block_sum_to<NEQ>(sq, A.npart + (size_t)blockIdx.x * NEQ);
 }
@@ -1348,14 +1364,12 @@ __device__ __forceinline__ double sutherland(const DevParams &P, double t) {
 template <typename R>
 __device__ __forceinline__ void store_state(const KArgs<R> &A, int i, const double *rec) {
     double *o = A.qn + (size_t)i * REC;
-    st4(o, rec);
-    st4(o + 4, rec + 4);
+    st8(o, rec);
     if (sizeof(R) == 4) {
         R s[REC];
 #pragma unroll
         for (int e = 0; e < REC; ++e) s[e] = R(rec[e]);
-        st4(A.qsn + (size_t)i * REC, s);
-        st4(A.qsn + (size_t)i * REC + 4, s + 4);
+        st8(A.qsn + (size_t)i * REC, s);
     }
 }
 
