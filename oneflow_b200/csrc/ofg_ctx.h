@@ -38,6 +38,8 @@ struct ofg_ctx {
     // ---- device ----
     cudaStream_t stream = nullptr;      // stream every launch goes to
     cudaStream_t ownStream = nullptr;   // the context's own stream (set when a caller's stream is in use)
+    cudaStream_t sideStream = nullptr;  // the iteration graph's branch (capture only)
+    cudaEvent_t forkEvent[2] = {nullptr, nullptr};
     int *d_lcb = nullptr, *d_bct = nullptr;                 // left cell and BC code of each boundary face
     int *d_nb_off = nullptr, *d_nbl = nullptr;              // per-cell neighbour lists (int2 pairs)
     int *d_lo_off = nullptr, *d_lol = nullptr, *d_up_off = nullptr, *d_upl = nullptr;
