@@ -1049,7 +1049,7 @@ int ofg_calc_boundary(ofg_ctx *c, int tid) {
 enum Fork { F_MAIN, F_FORK, F_SIDE, F_JOIN };   // a task of the chain; the branch's start, a task of it, its end
 struct Step { Fork where; int task; };
 static const Step kNsSteps[] = {{F_MAIN, T_ADVANCE}, {F_MAIN, T_P_GRADLIM}, {F_MAIN, T_P_FLUX}, {F_MAIN, T_P_FSUM},
-                                {F_FORK, 0}, {F_SIDE, T_NORM}, {F_MAIN, T_P_CLIP}, {F_MAIN, T_LOWER},
+                                {F_FORK, 0}, {F_SIDE, T_NORM}, {F_MAIN, T_CLIP0}, {F_MAIN, T_LOWER1},
                                 {F_MAIN, T_UPPER}, {F_MAIN, T_UPDATE}, {F_MAIN, T_BOUNDARY_NEXT}};
 static const Step kTurbSteps[] = {{F_MAIN, T_TURB_RHS}, {F_FORK, 0}, {F_SIDE, T_TURB_NORM}, {F_MAIN, T_TURB_LOWER},
                                   {F_MAIN, T_TURB_UPPER}, {F_MAIN, T_TURB_UPDATE}, {F_MAIN, T_TURB_BOUNDARY}};

@@ -107,7 +107,9 @@ enum Task {
     T_TURB_NORM_ONLY,
     // parts of T_TS_RES / T_TURB_RHS, timed separately by ofg_profile_step
     T_P_GRADLIM, T_P_FLUX, T_P_CLIP, T_P_TURB_GRAD, T_P_TURB_FLUX, T_P_FSUM,
-    T_FORCES, T_GRAD_ONLY, T_CALC_LHS
+    T_FORCES, T_GRAD_ONLY, T_CALC_LHS,
+    // the fused iteration's: on meshes where it pays the lower sweep's first level runs with the diagonal
+    T_CLIP0, T_LOWER1
 };
 int launch_task_f64(ofg_ctx *c, int task, cudaStream_t s);
 int launch_task_f32(ofg_ctx *c, int task, cudaStream_t s);

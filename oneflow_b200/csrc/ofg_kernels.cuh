@@ -227,25 +227,6 @@ __device__ __forceinline__ double face_vis_spec(const DevParams &P, const R *ql,
     return 0.0;
 }
 
-// UTimeStep::ModifyTimeStep / CalcLgTimeStep, then the diagonal of the
-// LU-SGS system for the sweeps: UNsSpectrum::CalcImplicitSpectrum
-// (sp2 = 1 for a steady solve), rad = (1/dt) vol + inviscid + viscous radius
-template <typename R>
-__global__ void __launch_bounds__(256) k_timestep_clip(KArgs<R> A) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= A.nCells) return;
-    double ts = A.dt[c];
-    if (A.P.timestepModel != 1) {
-        double mn = A.scal[S_MINDT];
-        if (A.P.timestepModel == 2) { ts = mn; A.dt[c] = ts; }
-        else if (A.P.max_time_ratio > 0) { ts = fmin(ts, A.P.max_time_ratio * mn); A.dt[c] = ts; }
-    }
-    double s = (1.0 / ts) * double(A.cgeo[(size_t)c * CGR + 3]);
-    s += A.invsr[c];
-    s += A.vissr[c];
-    A.rad[c] = s;
-}
-
 // ---------------------------------------------------------------------------
 // Gradients + limiter in one gather.  Gradients: CalcGradGGCellWeight
 // (codes/usolver/src/UGrad.cpp:88-149), the face-average Green-Gauss
@@ -1270,11 +1251,10 @@ __device__ __forceinline__ void sweep_rhs0(const KArgs<R> &A, int c, const int *
     }
 }
 
+// dq = (res - rhs0) / diag
 template <typename R>
-__device__ __forceinline__ void lusgs_lower_cell(const KArgs<R> &A, int c) {
-    double rhs0[NEQ] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    sweep_rhs0(A, c, A.lo_off, A.lol, rhs0);
-    const Divisor rad = make_divisor(A.rad[c]);
+__device__ __forceinline__ void lower_increment(const KArgs<R> &A, int c, const double *rhs0, double diag) {
+    const Divisor rad = make_divisor(diag);
     const double *rs = A.res + (size_t)c * NEQ;
     double y[NEQ], v[NEQ];
 #pragma unroll
@@ -1285,6 +1265,13 @@ __device__ __forceinline__ void lusgs_lower_cell(const KArgs<R> &A, int c) {
     for (int e = 0; e < NEQ; ++e) o[e] = R(v[e]);
     o[5] = o[6] = o[7] = R(0);
     st8(A.dq + (size_t)c * DQR, o);
+}
+
+template <typename R>
+__device__ __forceinline__ void lusgs_lower_cell(const KArgs<R> &A, int c) {
+    double rhs0[NEQ] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    sweep_rhs0(A, c, A.lo_off, A.lol, rhs0);
+    lower_increment(A, c, rhs0, A.rad[c]);
 }
 
 template <typename R>
@@ -1301,6 +1288,32 @@ __device__ __forceinline__ void lusgs_upper_cell(const KArgs<R> &A, int c) {
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) o[e] = R(v[e]);
     st8(A.dq + (size_t)c * DQR, o);
+}
+
+// UTimeStep::ModifyTimeStep / CalcLgTimeStep, then the diagonal of the
+// LU-SGS system for the sweeps: UNsSpectrum::CalcImplicitSpectrum
+// (sp2 = 1 for a steady solve), rad = (1/dt) vol + inviscid + viscous radius
+// LOWER0 (the fused iteration, after the residual): the cells without earlier
+// neighbours, the lower sweep's first level, take their increments here too
+// (first_level_early says where that pays).
+template <typename R, bool LOWER0 = false>
+__global__ void __launch_bounds__(256) k_timestep_clip(KArgs<R> A) {
+    int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= A.nCells) return;
+    double ts = A.dt[c];
+    if (A.P.timestepModel != 1) {
+        double mn = A.scal[S_MINDT];
+        if (A.P.timestepModel == 2) { ts = mn; A.dt[c] = ts; }
+        else if (A.P.max_time_ratio > 0) { ts = fmin(ts, A.P.max_time_ratio * mn); A.dt[c] = ts; }
+    }
+    double s = (1.0 / ts) * double(A.cgeo[(size_t)c * CGR + 3]);
+    s += A.invsr[c];
+    s += A.vissr[c];
+    A.rad[c] = s;
+    if (LOWER0 && A.lo_off[c] == A.lo_off[c + 1]) {
+        const double none[NEQ] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        lower_increment(A, c, none, s);
+    }
 }
 
 // one level of a sweep per launch (cells order[start .. start+count))

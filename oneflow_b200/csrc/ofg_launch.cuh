@@ -153,6 +153,13 @@ inline ChainPlan chain_plan(const ofg_ctx *c, bool lower) {
                      reinterpret_cast<const int2 *>(b.edge), b.cell, b.nlev, b.far, b.slots, c->chainStatus};
 }
 
+// Whether the fused iteration runs the NS lower sweep's first level with the
+// diagonal (k_timestep_clip): a launch fewer, but its blocks then write
+// increments colour by colour.  Measured, us an iteration
+// without / with: 4,096 cells 38.3 / 36.2, 113,886 84.9 / 82.2, 312,000 (FP64)
+// 624.2 / 622.4, 600,000 469.9 / 470.8, 768,640 631.6 / 634.2.
+inline bool first_level_early(const ofg_ctx *c) { return !chained(c) && c->nCells <= 400000; }
+
 template <typename K, typename... Args>
 int launch_chain(ofg_ctx *c, K one, K many, size_t smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg{};
@@ -235,16 +242,23 @@ int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
         if (task == T_TS_RES || task == T_P_CLIP) OFG_LAUNCH(k_timestep_clip<R>, nblk(N, 256), 256, s, A);
         break;
     }
+    case T_CLIP0: {
+        KArgs<R> A = make_args<R>(c, false);
+        if (first_level_early(c)) OFG_LAUNCH((k_timestep_clip<R, true>), nblk(N, 256), 256, s, A);
+        else OFG_LAUNCH(k_timestep_clip<R>, nblk(N, 256), 256, s, A);
+        break;
+    }
     case T_CALC_LHS: {   // CALC_LHS of the multi-stage scheme (same 128-cell blocks as the norm partials)
         KArgs<R> A = make_args<R>(c, false);
         OFG_LAUNCH(k_calc_lhs<R>, nblk(N, 128), 128, s, A, c->lhsCoef);
         break;
     }
-    case T_LOWER: {
+    case T_LOWER:
+    case T_LOWER1: {
         KArgs<R> A = make_args<R>(c, false);
         int nl = int(c->lowOff.size()) - 1;
         if (chained(c)) return launch_chain_ns<R, true>(c, A, s);
-        for (int l = 0; l < nl; ++l) {
+        for (int l = task == T_LOWER1 && first_level_early(c) ? 1 : 0; l < nl; ++l) {
             int st = c->lowOff[l], cnt = c->lowOff[l + 1] - st;
             const int *ord = (const int *)c->d_lowOrder;
             if constexpr (sizeof(R) == 4) {
