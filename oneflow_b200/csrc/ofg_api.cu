@@ -546,7 +546,7 @@ void ofg_destroy(ofg_ctx *c) {
                     c->d_lowOrder, c->d_upOrder, c->d_key, c->d_fgeo, c->d_cgeo, c->d_wdist, c->d_wall, c->d_wallG,
                     c->d_fgeoD, c->d_fofs, c->d_lr, c->d_fout,
                     c->d_q[0], c->d_q[1], c->d_qs[0], c->d_qs[1], c->d_res, c->d_dq, c->d_dt, c->d_invsr, c->d_vissr, c->d_rad,
-                    c->d_bcq, c->d_partial, c->d_npart, c->d_tpart, c->d_red, c->d_redCount, c->d_stage, c->d_scal, c->d_hist, c->d_gl, c->d_mm, c->d_fix,
+                    c->d_bcq, c->d_partial, c->d_npart, c->d_tpart, c->d_red, c->d_redCount, c->d_stage, c->d_scal, c->d_ext, c->d_hist, c->d_gl, c->d_mm, c->d_fix,
                     c->d_nut, c->d_dnut, c->d_resT, c->d_impsrT, c->d_matL, c->d_matR, c->d_thist, c->d_gnut};
     for (void *v : ptrs) if (v) cudaFree(v);
     free_chain(c);
@@ -741,6 +741,7 @@ int ofg_upload_mesh(ofg_ctx *c, int nNodes, const double *xN, const double *yN, 
     if ((rc = upload<unsigned int>(c, &c->d_redCount, nullptr, 1))) return rc;
     CK(cudaMemset(c->d_redCount, 0, sizeof(unsigned int)));
     if ((rc = upload<double>(c, &c->d_scal, nullptr, 32))) return rc;
+    if ((rc = upload<long long>(c, &c->d_ext, nullptr, 2 * NEQ))) return rc;
     c->histCap = 1 << 16;
     if ((rc = upload<double>(c, &c->d_hist, nullptr, (size_t)c->histCap * NEQ))) return rc;
     if ((rc = upload<int>(c, &c->d_fix, nullptr, 1 + c->fixcap))) return rc;
@@ -1048,9 +1049,9 @@ int ofg_calc_boundary(ofg_ctx *c, int tid) {
 // 467.0.  The CFL advance beside the gradients was not worth its fork and join.
 enum Fork { F_MAIN, F_FORK, F_SIDE, F_JOIN };   // a task of the chain; the branch's start, a task of it, its end
 struct Step { Fork where; int task; };
-static const Step kNsSteps[] = {{F_MAIN, T_ADVANCE}, {F_MAIN, T_P_GRADLIM}, {F_MAIN, T_P_FLUX}, {F_MAIN, T_P_FSUM},
+static const Step kNsSteps[] = {{F_MAIN, T_GRADLIM0}, {F_MAIN, T_P_FLUX}, {F_MAIN, T_P_FSUM},
                                 {F_FORK, 0}, {F_SIDE, T_NORM}, {F_MAIN, T_CLIP0}, {F_MAIN, T_LOWER1},
-                                {F_MAIN, T_UPPER}, {F_MAIN, T_UPDATE}, {F_MAIN, T_BOUNDARY_NEXT}};
+                                {F_MAIN, T_UPPER}, {F_MAIN, T_UPDATE_NEXT}, {F_MAIN, T_BOUNDARY_NEXT}};
 static const Step kTurbSteps[] = {{F_MAIN, T_TURB_RHS}, {F_FORK, 0}, {F_SIDE, T_TURB_NORM}, {F_MAIN, T_TURB_LOWER},
                                   {F_MAIN, T_TURB_UPPER}, {F_MAIN, T_TURB_UPDATE}, {F_MAIN, T_TURB_BOUNDARY}};
 
@@ -1085,6 +1086,8 @@ static int prepare_steps(ofg_ctx *c, int nsteps) {
     double sc[4] = {double(c->outerSteps), double(c->outerSteps), 0.0, double(c->outerSteps)};
     CK(cudaMemcpyAsync(c->d_scal + S_STEP, sc, 2 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->d_scal + S_THISTN, sc + 3, sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    // an LU-SGS iteration starts the step after it; the first one is started here
+    if (!multi_stage(c) && (rc = launch(c, T_ADVANCE))) return rc;
     return sync(c);
 }
 

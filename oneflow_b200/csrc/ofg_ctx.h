@@ -69,6 +69,7 @@ struct ofg_ctx {
     void *d_dq = nullptr;                                   // [nCells][DQR] at the face precision
     double *d_stage = nullptr;                              // [5][nT] state transfer staging (on first use)
     double *d_bcq = nullptr, *d_partial = nullptr, *d_scal = nullptr, *d_hist = nullptr;
+    long long *d_ext = nullptr;                             // limiter extremes (see KArgs::ext)
     double *d_npart = nullptr, *d_tpart = nullptr;          // per-block sums of squares of the residuals
     double *d_red = nullptr;                                // [kRedBlocks][5] block sums of the grid reductions
     unsigned int *d_redCount = nullptr;                     // their ticket counter (0 between launches)
@@ -108,8 +109,9 @@ enum Task {
     // parts of T_TS_RES / T_TURB_RHS, timed separately by ofg_profile_step
     T_P_GRADLIM, T_P_FLUX, T_P_CLIP, T_P_TURB_GRAD, T_P_TURB_FLUX, T_P_FSUM,
     T_FORCES, T_GRAD_ONLY, T_CALC_LHS,
-    // the fused iteration's: on meshes where it pays the lower sweep's first level runs with the diagonal
-    T_CLIP0, T_LOWER1
+    // the fused iteration's: on meshes where it pays the lower sweep's first
+    // level runs with the diagonal; the update starts the next outer step
+    T_CLIP0, T_LOWER1, T_UPDATE_NEXT, T_GRADLIM0
 };
 int launch_task_f64(ofg_ctx *c, int task, cudaStream_t s);
 int launch_task_f32(ofg_ctx *c, int task, cudaStream_t s);

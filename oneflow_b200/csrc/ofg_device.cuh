@@ -60,9 +60,9 @@ constexpr int FOR = 6;    // face-pass record (mixed path): flux[5] FP64, then t
                           // spectral radii as two FP32 values in the sixth slot (48 B, three 16-B words)
 constexpr int FOFS = 8;   // face-local offsets record (mixed path), FP32
 
-// slots of the small device scalar array (cfl, min dt, limiter eps, norms,
+// slots of the small device scalar array (cfl, min dt, norms,
 // outer-step counter, residual-history length)
-enum { S_CFL = 0, S_MINDT = 1, S_EPS = 2 /* 5 slots */, S_NORM = 8 /* 5 slots */, S_STEP = 14, S_HISTN = 15,
+enum { S_CFL = 0, S_MINDT = 1, S_NORM = 8 /* 5 slots */, S_STEP = 14, S_HISTN = 15,
        S_TNORM = 16, S_THISTN = 17, S_FORCE = 20 /* 9 slots: total, pressure, viscous force */, S_NSCAL = 29 };
 
 enum BcCode { BC_EXTRAP = 1, BC_SOLID = 2, BC_SYM = 3, BC_FAR = 4, BC_INFLOW = 5, BC_OUTFLOW = 6 };

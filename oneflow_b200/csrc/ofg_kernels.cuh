@@ -38,7 +38,8 @@ struct KArgs {
     R *dq;                                 // [nCells][DQR] LU-SGS increments (whole sectors per cell)
     R *gl;                                 // [nCells][GLR]
     R *mm;                                 // [nCells][MMR]
-    double *partial, *scal;
+    double *scal;
+    long long *ext;                        // zone-wide limiter extremes: least minima, then largest maxima, as ordered keys
     double *npart, *tpart;                 // per-block sums of squares of res / resT (128-cell blocks)
     double *red; unsigned int *redCount;   // block sums and ticket of the grid reductions
     int *fixlist; int fixcap;
@@ -237,6 +238,22 @@ __device__ __forceinline__ double face_vis_spec(const DevParams &P, const R *ql,
 // Venkatakrishnan with eps^2 = (K h)^3), 2 min/max and block extremes for the
 // zone-wide Venkatakrishnan eps (limiter in k_limiter_global).
 // ---------------------------------------------------------------------------
+// doubles as integers of the same order, for integer atomics: the extremes of
+// the blocks are exact in any order, and each block of k_limiter_global forms
+// the eps from them (a kernel of one block between the two took 5.9 us over 890
+// blocks' extremes, 9.7 over 2,440)
+__device__ __forceinline__ long long ordered_key(double v) {
+    const long long b = __double_as_longlong(v);
+    return b >= 0 ? b : b ^ 0x7fffffffffffffffll;
+}
+__device__ __forceinline__ double from_key(long long k) {
+    return __longlong_as_double(k >= 0 ? k : k ^ 0x7fffffffffffffffll);
+}
+// no extremes yet (before a gradient pass with the zone-wide eps)
+__device__ __forceinline__ void clear_extremes(long long *ext) {
+    for (int e = 0; e < NEQ; ++e) { ext[e] = ordered_key(1.0e40); ext[NEQ + e] = ordered_key(-1.0e40); }
+}
+
 template <typename R>
 __device__ __forceinline__ R barth_fn(R dqv, R minv, R maxv, R dot) {
     if (dot < R(0)) return R(0);
@@ -497,48 +514,25 @@ __global__ void __launch_bounds__(128, MINB) k_gradlim(KArgs<R> A, int nvar, int
             }
             __syncthreads();
         }
-        if (threadIdx.x == 0) {
-#pragma unroll
-            for (int e = 0; e < 2 * NEQ; ++e) A.partial[(size_t)blockIdx.x * 10 + e] = sred[e][0];
-        }
-    }
-}
-
-// zone-wide eps per equation, ULimiter.cpp:571-593 (single block; min/max exact)
-template <typename R>
-__global__ void __launch_bounds__(256) k_limiter_eps(KArgs<R> A, int nPartial) {
-    __shared__ double smn[NEQ][256], smx[NEQ][256];
-    double lmin[NEQ], lmax[NEQ];
-#pragma unroll
-    for (int e = 0; e < NEQ; ++e) { lmin[e] = 1.0e40; lmax[e] = -1.0e40; }
-    for (int i = threadIdx.x; i < nPartial; i += blockDim.x)
-#pragma unroll
-        for (int e = 0; e < NEQ; ++e) {
-            lmin[e] = fmin(lmin[e], A.partial[(size_t)i * 10 + e]);
-            lmax[e] = fmax(lmax[e], A.partial[(size_t)i * 10 + 5 + e]);
-        }
-#pragma unroll
-    for (int e = 0; e < NEQ; ++e) { smn[e][threadIdx.x] = lmin[e]; smx[e][threadIdx.x] = lmax[e]; }
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s)
-#pragma unroll
-            for (int e = 0; e < NEQ; ++e) {
-                smn[e][threadIdx.x] = fmin(smn[e][threadIdx.x], smn[e][threadIdx.x + s]);
-                smx[e][threadIdx.x] = fmax(smx[e][threadIdx.x], smx[e][threadIdx.x + s]);
+        if (threadIdx.x < 2 * NEQ) {
+            const double v = sred[threadIdx.x][0];
+            if (v == v) {
+                if (threadIdx.x < NEQ) atomicMin(A.ext + threadIdx.x, ordered_key(v));
+                else atomicMax(A.ext + threadIdx.x, ordered_key(v));
             }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int e = 0; e < NEQ; ++e) {
-            double eps = A.P.vencat_coef * fmax(smx[e][0] - smn[e][0], 1.0);
-            A.scal[S_EPS + e] = eps * eps + SMALLD;
         }
+    }
 }
 
 template <typename R>
 __global__ void __launch_bounds__(128) k_limiter_global(KArgs<R> A) {
+    // zone-wide eps per equation, ULimiter.cpp:571-593
+    __shared__ double seps[NEQ];
+    if (threadIdx.x < NEQ) {
+        const double e = A.P.vencat_coef * fmax(from_key(A.ext[NEQ + threadIdx.x]) - from_key(A.ext[threadIdx.x]), 1.0);
+        seps[threadIdx.x] = e * e + SMALLD;
+    }
+    __syncthreads();
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= A.nCells) return;
     R cgc[CGR], rec[GLR];
@@ -548,7 +542,7 @@ __global__ void __launch_bounds__(128) k_limiter_global(KArgs<R> A) {
     const R *m = A.mm + (size_t)c * MMR;
     R mn[NEQ], mx[NEQ], eps[NEQ], lim[NEQ];
 #pragma unroll
-    for (int e = 0; e < NEQ; ++e) { mn[e] = m[e]; mx[e] = m[5 + e]; eps[e] = R(A.scal[S_EPS + e]); }
+    for (int e = 0; e < NEQ; ++e) { mn[e] = m[e]; mx[e] = m[5 + e]; eps[e] = R(seps[e]); }
     cell_limiter(A, c, cgc, rec, mn, mx, eps, lim);
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) o[18 + e] = lim[e];
@@ -1478,13 +1472,32 @@ __global__ void __launch_bounds__(256) k_update(KArgs<R> A) {
     update_cell(A, c, dd);
 }
 
+// CFL ramp (TimeStep::CalcCfl, codes/ns/src/TimeStep.cpp:43-59) of outer step
+// `it`; also resets the zone-wide minimum time step that the residual kernel's
+// blocks lower, and the limiter extremes that the gradient kernel's widen.
+struct Ramp { double cflst, cfled; int ncfl; };
+__device__ __forceinline__ void start_step(double *scal, long long *ext, double it, const Ramp &r) {
+    scal[S_MINDT] = 1.0e40;
+    scal[S_STEP] = it;
+    double cfl = r.cfled;
+    if (it < r.ncfl) {
+        double delta = (r.cfled - r.cflst) / r.ncfl;
+        cfl = r.cflst + delta * it;
+    }
+    scal[S_CFL] = cfl;
+    clear_extremes(ext);
+}
+
 // UNsUpdate::SolutionFix (codes/uns/src/UNsUpdate.cpp:94-133) for the cells
 // that failed every positivity retry.  The reference updates in place in its
 // sweep order, so a neighbour earlier in that order contributes its new value
 // and a later one its old value; one thread replays that order.
-template <typename R>
-__global__ void k_solution_fix(KArgs<R> A) {
+// NEXT (the fused iteration): then starts the next outer step, which nothing
+// between here and its gradients reads (a launch of its own took 1.7 us).
+template <typename R, bool NEXT = false>
+__global__ void k_solution_fix(KArgs<R> A, Ramp ramp) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    if (NEXT) start_step(A.scal, A.ext, A.scal[S_STEP] + 1.0, ramp);
     int n = A.fixlist[0];
     if (n <= 0) return;
     if (n > A.fixcap) n = A.fixcap;

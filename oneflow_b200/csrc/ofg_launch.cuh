@@ -11,20 +11,14 @@
 
 namespace ofg {
 
-// CFL ramp (TimeStep::CalcCfl, codes/ns/src/TimeStep.cpp:43-59).  step < 0:
-// advance the device-side outer-step counter first (graph path).  Also resets
-// the zone-wide minimum time step that the residual kernel's blocks lower.
-static __global__ void k_cfl(double *scal, double step, double cflst, double cfled, int ncfl) {
+// step < 0: the device-side outer-step counter's next step
+static __global__ void k_cfl(double *scal, long long *ext, double step, Ramp ramp) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    scal[S_MINDT] = 1.0e40;
-    double it = step;
-    if (step < 0) { scal[S_STEP] += 1.0; it = scal[S_STEP]; } else { scal[S_STEP] = step; }
-    double cfl = cfled;
-    if (it < ncfl) {
-        double delta = (cfled - cflst) / ncfl;
-        cfl = cflst + delta * it;
-    }
-    scal[S_CFL] = cfl;
+    start_step(scal, ext, step < 0 ? scal[S_STEP] + 1.0 : step, ramp);
+}
+
+static __global__ void k_clear_extremes(long long *ext) {
+    if (threadIdx.x == 0) clear_extremes(ext);
 }
 
 static __global__ void k_norm_hist(double *scal, double *hist, int cap) {
@@ -60,7 +54,7 @@ KArgs<R> make_args(ofg_ctx *c, bool onCurrent) {
     A.res = c->d_res; A.dq = static_cast<R *>(c->d_dq); A.dt = c->d_dt; A.invsr = c->d_invsr; A.vissr = c->d_vissr;
     A.rad = c->d_rad;
     A.bcq = c->d_bcq; A.gl = static_cast<R *>(c->d_gl); A.mm = static_cast<R *>(c->d_mm);
-    A.partial = c->d_partial; A.scal = c->d_scal; A.fixlist = c->d_fix; A.fixcap = c->fixcap;
+    A.scal = c->d_scal; A.ext = c->d_ext; A.fixlist = c->d_fix; A.fixcap = c->fixcap;
     A.npart = c->d_npart; A.tpart = c->d_tpart; A.red = c->d_red; A.redCount = c->d_redCount;
     A.nut = c->d_nut; A.dnut = c->d_dnut; A.resT = c->d_resT; A.impsrT = c->d_impsrT;
     A.matL = c->d_matL; A.matR = c->d_matR; A.gnut = static_cast<R *>(c->d_gnut);
@@ -75,9 +69,11 @@ inline int nblk(long long n, int b) { return int((n + b - 1) / b); }
         ++c->launches;                                                     \
     } while (0)
 
-// gradients and limiter of the current state (UPDATE_RESIDUALS' first half)
+// gradients and limiter of the current state (UPDATE_RESIDUALS' first half);
+// started: the outer step's start has cleared the limiter extremes, and no
+// gradient pass since has widened them
 template <typename R>
-void launch_gradlim(ofg_ctx *c, const KArgs<R> &A, cudaStream_t s) {
+void launch_gradlim(ofg_ctx *c, const KArgs<R> &A, cudaStream_t s, bool started = false) {
     const int N = c->nCells;
     bool needGrad = c->p.ilim != -1 || c->p.vismodel > 0;
     if (!needGrad) return;
@@ -85,6 +81,7 @@ void launch_gradlim(ofg_ctx *c, const KArgs<R> &A, cudaStream_t s) {
     bool venkatGlobal = c->p.ilim == 2 && !c->p.venkat_kh3;
     int limMode = (c->p.ilim == 1 || c->p.ilim == 2) ? (venkatGlobal ? 2 : 1) : 0;
     int nb = nblk(N, 128);
+    if (limMode == 2 && !started) OFG_LAUNCH(k_clear_extremes, 1, 32, s, A.ext);
     if constexpr (sizeof(R) == 4) {
         const int gb = c->tune.grad_block == 64 ? 64 : 128;   // the limiter's block extremes are exact either way
         nb = nblk(N, gb);
@@ -96,10 +93,7 @@ void launch_gradlim(ofg_ctx *c, const KArgs<R> &A, cudaStream_t s) {
     } else {
         OFG_LAUNCH(k_gradlim<R>, nb, 128, s, A, nvar, limMode);
     }
-    if (limMode == 2) {
-        OFG_LAUNCH(k_limiter_eps<R>, 1, 256, s, A, nb);
-        OFG_LAUNCH(k_limiter_global<R>, nb, 128, s, A);
-    }
+    if (limMode == 2) OFG_LAUNCH(k_limiter_global<R>, nblk(N, 128), 128, s, A);
 }
 
 // The flux / time-step pass of MODE (as k_residual): the FP64 path's
@@ -208,13 +202,14 @@ int launch_chain_sa(ofg_ctx *c, const KArgs<R> &A, cudaStream_t s) {
 template <typename R>
 int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
     const int N = c->nCells;
+    const Ramp ramp{c->p.cflst, c->p.cfled, c->p.ncfl};
     switch (task) {
     case T_CFL: {
-        OFG_LAUNCH(k_cfl, 1, 32, s, c->d_scal, double(c->outerSteps), c->p.cflst, c->p.cfled, c->p.ncfl);
+        OFG_LAUNCH(k_cfl, 1, 32, s, c->d_scal, c->d_ext, double(c->outerSteps), ramp);
         break;
     }
     case T_ADVANCE: {
-        OFG_LAUNCH(k_cfl, 1, 32, s, c->d_scal, -1.0, c->p.cflst, c->p.cfled, c->p.ncfl);
+        OFG_LAUNCH(k_cfl, 1, 32, s, c->d_scal, c->d_ext, -1.0, ramp);
         break;
     }
     case T_TIMESTEP: {   // CALC_TIME_STEP alone (after T_CFL, which resets the minimum)
@@ -230,12 +225,13 @@ int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
         break;
     }
     case T_TS_RES:       // CALC_TIME_STEP + LOAD_RESIDUALS + UPDATE_RESIDUALS in one gather
-    case T_P_GRADLIM:    // (its three parts, launched separately by the profiler)
+    case T_P_GRADLIM:    // (its parts, launched separately by the profiler and the fused iteration)
+    case T_GRADLIM0:
     case T_P_FLUX:
     case T_P_FSUM:
     case T_P_CLIP: {
         KArgs<R> A = make_args<R>(c, false);
-        if (task == T_TS_RES || task == T_P_GRADLIM) launch_gradlim<R>(c, A, s);
+        if (task == T_TS_RES || task == T_P_GRADLIM || task == T_GRADLIM0) launch_gradlim<R>(c, A, s, task == T_GRADLIM0);
         if (task == T_TS_RES) launch_flux<R, 0>(c, A, s);
         if (task == T_P_FLUX) launch_flux<R, 0>(c, A, s, 1);
         if (task == T_P_FSUM) launch_flux<R, 0>(c, A, s, 2);
@@ -297,10 +293,12 @@ int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
         }
         break;
     }
-    case T_UPDATE: {
+    case T_UPDATE:
+    case T_UPDATE_NEXT: {
         KArgs<R> A = make_args<R>(c, false);
         OFG_LAUNCH(k_update<R>, nblk(N, 256), 256, s, A);
-        OFG_LAUNCH(k_solution_fix<R>, 1, 32, s, A);
+        if (task == T_UPDATE_NEXT) OFG_LAUNCH((k_solution_fix<R, true>), 1, 32, s, A, ramp);
+        else OFG_LAUNCH(k_solution_fix<R>, 1, 32, s, A, ramp);
         break;
     }
     case T_BOUNDARY_NEXT: {
