@@ -1189,9 +1189,10 @@ __device__ __forceinline__ void edge_coef(const DevParams &P, const R *qa, const
 __device__ __forceinline__ double sum2(double a, double b, double c, double d) { return a * b + c * d; }
 __device__ __forceinline__ float sum2(float a, float b, float c, float d) { return __fmaf_rn(c, d, __fmul_rn(a, b)); }
 
-// The neighbour's increment dqj through the coefficients, added to rhs0
+// The neighbour's increment dqj through the coefficients: its flux increment df
+// and viscous part vd (vismodel > 0)
 template <typename R>
-__device__ __forceinline__ void edge_apply(const DevParams &P, const EdgeCoef<R> &E, const R *dqj, double *rhs0) {
+__device__ __forceinline__ void edge_terms(const DevParams &P, const EdgeCoef<R> &E, const R *dqj, R *df, R *vd) {
     R d0 = R(dqj[0]), d1 = R(dqj[1]), d2 = R(dqj[2]), d3 = R(dqj[3]), d4 = R(dqj[4]);
     R dc = E.vn * d0 - E.xn * d1 - E.yn * d2 - E.zn * d3;
     R c2dc = E.c2 * dc;
@@ -1200,7 +1201,6 @@ __device__ __forceinline__ void edge_apply(const DevParams &P, const EdgeCoef<R>
     dh += E.af * d0;
     R term1 = sum2(dh, E.x1, dc, E.x2);
     R term2 = sum2(c2dc, E.x1, dh, E.x2);
-    R df[NEQ];
     df[0] = E.lmd1 * d0 - term1;
     df[1] = E.lmd1 * d1 - E.u * term1 + E.xn * term2;
     df[2] = E.lmd1 * d2 - E.v * term1 + E.yn * term2;
@@ -1209,8 +1209,18 @@ __device__ __forceinline__ void edge_apply(const DevParams &P, const EdgeCoef<R>
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) df[e] *= E.fa;
     if (P.vismodel > 0) {
-        rhs0[0] -= double(E.visrad * d0); rhs0[1] -= double(E.visrad * d1); rhs0[2] -= double(E.visrad * d2);
-        rhs0[3] -= double(E.visrad * d3); rhs0[4] -= double(E.visrad * d4);
+        vd[0] = E.visrad * d0; vd[1] = E.visrad * d1; vd[2] = E.visrad * d2; vd[3] = E.visrad * d3; vd[4] = E.visrad * d4;
+    }
+}
+
+// the same, added to rhs0
+template <typename R>
+__device__ __forceinline__ void edge_apply(const DevParams &P, const EdgeCoef<R> &E, const R *dqj, double *rhs0) {
+    R df[NEQ], vd[NEQ];
+    edge_terms(P, E, dqj, df, vd);
+    if (P.vismodel > 0) {
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) rhs0[e] -= double(vd[e]);
     }
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) rhs0[e] += double(df[e]);
@@ -1245,6 +1255,47 @@ __device__ __forceinline__ void sweep_rhs0(const KArgs<R> &A, int c, const int *
     }
 }
 
+// sweep_rhs0 by four lanes a cell, a face each at a time (they hold the same
+// result): a face's serial chain of FP64 quotients and roots, about 2,000
+// cycles, once for four faces; the terms are added in the faces' order.
+template <typename R>
+__device__ __forceinline__ void sweep_rhs0_quad(const KArgs<R> &A, int c, bool active, const int *off, const int2 *list,
+                                                double *rhs0) {
+    const int j = threadIdx.x & 3;
+    const int kb = active ? off[c] : 0, ke = active ? off[c + 1] : 0;
+    R qc[REC];
+    if (kb < ke) ld8(A.qs + (size_t)c * REC, qc);
+    for (int k0 = kb; __any_sync(0xffffffffu, k0 < ke); k0 += 4) {
+        R df[NEQ] = {}, vd[NEQ] = {};
+        if (k0 + j < ke) {
+            const int2 e2 = __ldg(&list[k0 + j]);
+            const int f = nb_face(e2), nb = e2.y;
+            R qn[REC], fg[FGR], dqj[DQR];
+            ld8(A.qs + (size_t)nb * REC, qn);
+            ld8(A.fgeo + (size_t)f * FGR, fg);
+            ld8(A.dq + (size_t)nb * DQR, dqj);
+            R volb = A.P.visSRModel == 1 ? A.cgeo[(size_t)nb * CGR + 3] : R(1);
+            R xn = fg[0], yn = fg[1], zn = fg[2];
+            if (nb_right(e2)) { xn = -xn; yn = -yn; zn = -zn; }
+            EdgeCoef<R> E;
+            edge_coef(A.P, qc, qn, xn, yn, zn, fg[3], fg[7], volb, E);
+            edge_terms(A.P, E, dqj, df, vd);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool add = k0 + q < ke;
+#pragma unroll
+            for (int e = 0; e < NEQ; ++e) {
+                const double v = double(__shfl_sync(0xffffffffu, vd[e], q, 4)), f = double(__shfl_sync(0xffffffffu, df[e], q, 4));
+                double t = rhs0[e];
+                if (A.P.vismodel > 0) t -= v;
+                t += f;
+                rhs0[e] = add ? t : rhs0[e];
+            }
+        }
+    }
+}
+
 // dq = (res - rhs0) / diag
 template <typename R>
 __device__ __forceinline__ void lower_increment(const KArgs<R> &A, int c, const double *rhs0, double diag) {
@@ -1268,13 +1319,12 @@ __device__ __forceinline__ void lusgs_lower_cell(const KArgs<R> &A, int c) {
     lower_increment(A, c, rhs0, A.rad[c]);
 }
 
+// its lower-sweep increment less rhs0 / diag
 template <typename R>
-__device__ __forceinline__ void lusgs_upper_cell(const KArgs<R> &A, int c) {
-    double rhs0[NEQ] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    sweep_rhs0(A, c, A.up_off, A.upl, rhs0);   // ghost increments are zero: boundary faces not listed
+__device__ __forceinline__ void upper_increment(const KArgs<R> &A, int c, const double *rhs0) {
     const Divisor rad = make_divisor(A.rad[c]);
     R o[DQR];
-    ldp8(A.dq + (size_t)c * DQR, o);   // its own lower-sweep increment, rewritten below
+    ldp8(A.dq + (size_t)c * DQR, o);
     double v[NEQ];
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) v[e] = double(o[e]);
@@ -1282,6 +1332,13 @@ __device__ __forceinline__ void lusgs_upper_cell(const KArgs<R> &A, int c) {
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) o[e] = R(v[e]);
     st8(A.dq + (size_t)c * DQR, o);
+}
+
+template <typename R>
+__device__ __forceinline__ void lusgs_upper_cell(const KArgs<R> &A, int c) {
+    double rhs0[NEQ] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    sweep_rhs0(A, c, A.up_off, A.upl, rhs0);   // ghost increments are zero: boundary faces not listed
+    upper_increment(A, c, rhs0);
 }
 
 // UTimeStep::ModifyTimeStep / CalcLgTimeStep, then the diagonal of the
@@ -1321,6 +1378,19 @@ template <typename R, int MINB = MinBlocks<R>::sw>
 __global__ void __launch_bounds__(128, MINB) k_lusgs_upper(KArgs<R> A, const int *order, int start, int count) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < count) lusgs_upper_cell(A, order[start + t]);
+}
+
+// the same with four lanes a cell
+template <typename R, bool LOWER>
+__global__ void __launch_bounds__(128) k_lusgs_quad(KArgs<R> A, const int *order, int start, int count) {
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+    const bool active = t < count;
+    const int c = active ? order[start + t] : 0;
+    double rhs0[NEQ] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    sweep_rhs0_quad(A, c, active, LOWER ? A.lo_off : A.up_off, LOWER ? A.lol : A.upl, rhs0);
+    if (!active || (threadIdx.x & 3)) return;
+    if (LOWER) lower_increment(A, c, rhs0, A.rad[c]);
+    else upper_increment(A, c, rhs0);
 }
 
 // ---------------------------------------------------------------------------

@@ -147,6 +147,13 @@ inline ChainPlan chain_plan(const ofg_ctx *c, bool lower) {
                      reinterpret_cast<const int2 *>(b.edge), b.cell, b.nlev, b.far, b.slots, c->chainStatus};
 }
 
+// Whether an FP64 sweep level runs with four lanes a cell: as long as that
+// still leaves the SMs room.  Measured, us an iteration with a thread a cell /
+// four lanes: levels of 288 cells 33.3 / 29.2, 2,048 35.3 / 31.4, 8,192 35.3 / 32.1,
+// 18,432 37.4 / 35.3, 14,400 tetrahedra (SA) 203 / 193; of 32,768 46.1 / 51.2.
+// (The mixed path's approximate quotients and roots leave no such chain.)
+inline bool quad_level(int cells) { return cells <= 20000; }
+
 // Whether the fused iteration runs the NS lower sweep's first level with the
 // diagonal (k_timestep_clip): a launch fewer, but its blocks then write
 // increments colour by colour.  Measured, us an iteration
@@ -265,7 +272,8 @@ int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
                 default: OFG_LAUNCH((k_lusgs_lower<R, 8>), nblk(cnt, bs), bs, s, A, ord, st, cnt); break;
                 }
             } else {
-                OFG_LAUNCH(k_lusgs_lower<R>, nblk(cnt, 128), 128, s, A, ord, st, cnt);
+                if (quad_level(cnt)) OFG_LAUNCH((k_lusgs_quad<R, true>), nblk(4LL * cnt, 128), 128, s, A, ord, st, cnt);
+                else OFG_LAUNCH(k_lusgs_lower<R>, nblk(cnt, 128), 128, s, A, ord, st, cnt);
             }
         }
         break;
@@ -288,7 +296,8 @@ int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
                 default: OFG_LAUNCH((k_lusgs_upper<R, 8>), nblk(cnt, bs), bs, s, A, ord, st, cnt); break;
                 }
             } else {
-                OFG_LAUNCH(k_lusgs_upper<R>, nblk(cnt, 128), 128, s, A, ord, st, cnt);
+                if (quad_level(cnt)) OFG_LAUNCH((k_lusgs_quad<R, false>), nblk(4LL * cnt, 128), 128, s, A, ord, st, cnt);
+                else OFG_LAUNCH(k_lusgs_upper<R>, nblk(cnt, 128), 128, s, A, ord, st, cnt);
             }
         }
         break;
