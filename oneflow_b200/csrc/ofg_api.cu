@@ -10,6 +10,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "ofg_ctx.h"
@@ -271,12 +272,9 @@ bool chain_pays(const ofg_ctx *c) {
 }
 
 void free_chain(ofg_ctx *c) {
-    for (ChainBuf &b : c->chain) {
-        for (int *p : {b.lev, b.ref, b.edge, b.cell}) cudaFree(p);
-        b = ChainBuf();
-    }
-    cudaFree(c->d_chainCoef);
-    cudaFree(c->d_chainCell);
+    cudaFree(c->d_chain);   // holds both plans
+    c->d_chain = nullptr;
+    c->chain[0] = c->chain[1] = ChainBuf();
     c->d_chainCoef = nullptr;
     c->d_chainCell = nullptr;
 }
@@ -313,9 +311,6 @@ void build_lists(const ofg_ctx *c, NbLists &L) {
     }
 }
 
-template <typename T> int upload(ofg_ctx *c, T **d, const T *h, size_t n);
-int upload_bytes(ofg_ctx *c, void **d, const void *h, size_t bytes);
-
 // The chained sweeps' schedules (ofg_chain.cuh): edge slots [level][j-th edge][cell of the level], each edge with
 // its neighbour's place in the ring, or ~neighbour where the ring no longer (or not for the whole level) holds it.
 // Without the memory for them, or where a level is wider than the cluster's
@@ -331,15 +326,21 @@ int build_chain(ofg_ctx *c, const NbLists *lists = nullptr) {
         build_lists(c, own);
         lists = &own;
     }
-    long long most = 1;
-    std::vector<int> lev, ref, edge, cell, pos(c->nCells), at(c->nCells);
-    for (int dir = 0; dir < 2; ++dir) {
+    // the two sweeps' plans side by side
+    struct Plan {
+        std::vector<int> lev, ref, edge;
+        long long slots = 0;
+        int far = 0;
+        bool fits = true;
+    } plans[2];
+    auto build = [&](int dir) {
+        Plan &P = plans[dir];
         const std::vector<int> &order = dir == 0 ? c->lowOrder : c->upOrder, &off = dir == 0 ? c->lowOff : c->upOff;
         const std::vector<int> &nbOff = dir == 0 ? lists->loOff : lists->upOff;
         const std::vector<int> &nbl = dir == 0 ? lists->lol : lists->upl;
         const int nlev = int(off.size()) - 1;
-        lev.assign(4 * (size_t)nlev, 0);
-        long long slots = 0;
+        std::vector<int> pos(c->nCells), at(c->nCells);
+        P.lev.assign(4 * (size_t)nlev, 0);
         for (int l = 0; l < nlev; ++l) {
             int deg = 0;
             for (int k = off[l]; k < off[l + 1]; ++k) {
@@ -347,48 +348,79 @@ int build_chain(ofg_ctx *c, const NbLists *lists = nullptr) {
                 pos[i] = k; at[i] = l;
                 deg = std::max(deg, nbOff[i + 1] - nbOff[i]);
             }
-            int *m = &lev[4 * (size_t)l];
-            m[0] = off[l]; m[1] = off[l + 1] - off[l]; m[2] = int(slots); m[3] = deg;
-            slots += (long long)deg * m[1];
-            if (slots > INT32_MAX || m[1] > kChainLevel) { free_chain(c); return OFG_OK; }
+            int *m = &P.lev[4 * (size_t)l];
+            m[0] = off[l]; m[1] = off[l + 1] - off[l]; m[2] = int(P.slots); m[3] = deg;
+            P.slots += (long long)deg * m[1];
+            P.fits = P.fits && P.slots <= INT32_MAX / 4 && m[1] <= kChainLevel;
+            if (!P.fits) return;
         }
-        ref.assign(slots, kChainNone); edge.assign(2 * slots, -1); cell.assign(slots, 0);
-        int far = 0;
+        P.ref.assign(P.slots, kChainNone);
+        P.edge.assign(4 * P.slots, -1);
         for (int l = 0; l < nlev; ++l) {
-            const int *m = &lev[4 * (size_t)l];
+            const int *m = &P.lev[4 * (size_t)l];
             for (int t = 0; t < m[1]; ++t) {
                 const int i = order[m[0] + t];
                 size_t s = (size_t)m[2] + t;
                 for (int q = nbOff[i]; q < nbOff[i + 1]; ++q, s += m[1]) {   // ascending face id
                     const int nb = nbl[2 * (size_t)q + 1];
                     const bool near = pos[nb] + kChainRing >= off[l + 1];
-                    ref[s] = near ? pos[nb] & (kChainRing - 1) : ~nb;
+                    P.ref[s] = near ? pos[nb] & (kChainRing - 1) : ~nb;
                     // a global copy written after its signal is safe to read
                     // from the level after its warp's next signal on
-                    if (!near) far = std::max(far, l <= at[nb] + kChainGroups ? 2 : 1);
-                    edge[2 * s] = nbl[2 * (size_t)q];
-                    edge[2 * s + 1] = nb;
-                    cell[s] = i;
+                    if (!near) P.far = std::max(P.far, l <= at[nb] + kChainGroups ? 2 : 1);
+                    int *e = &P.edge[4 * s];
+                    e[0] = nbl[2 * (size_t)q]; e[1] = nb; e[2] = i;
                 }
             }
         }
-        ChainBuf &b = c->chain[dir];
-        b.nlev = nlev; b.slots = slots; b.far = far;
-        most = std::max(most, slots);
-        int rc = upload(c, &b.lev, lev.data(), lev.size());
-        if (!rc) rc = upload(c, &b.ref, ref.data(), ref.size());
-        if (!rc) rc = upload(c, &b.edge, edge.data(), edge.size());
-        if (!rc) rc = upload(c, &b.cell, cell.data(), cell.size());
-        if (!rc && dir == 1)
-            rc = upload_bytes(c, &c->d_chainCoef, nullptr, (size_t)most * kEdgeCoefs *
-                              (c->p.precision == OFG_PREC_MIXED ? sizeof(float) : sizeof(double)));
-        if (!rc && dir == 1) rc = upload(c, &c->d_chainCell, (const double *)nullptr, (size_t)kChainCell * c->nCells);
-        if (rc) {
-            cudaGetLastError();
-            free_chain(c);
-            return OFG_OK;
+    };
+    auto guarded = [&](int dir) {   // no memory for a plan: no chain
+        try {
+            build(dir);
+        } catch (const std::exception &) {
+            plans[dir].fits = false;
         }
+    };
+    std::thread lower;
+    try {
+        lower = std::thread(guarded, 0);
+    } catch (const std::exception &) {   // no thread: one after the other
     }
+    guarded(1);
+    if (lower.joinable()) lower.join();
+    else guarded(0);
+    if (!plans[0].fits || !plans[1].fits) return OFG_OK;
+    // one allocation: each plan's levels, edges and ring slots, then the sweep's scratch
+    const size_t real = c->p.precision == OFG_PREC_MIXED ? sizeof(float) : sizeof(double);
+    auto whole = [](size_t n) { return (n + 255) / 256 * 256; };
+    size_t at[2][3], n = 0;
+    for (int dir = 0; dir < 2; ++dir) {
+        const Plan &P = plans[dir];
+        const size_t sizes[3] = {P.lev.size(), P.edge.size(), P.ref.size()};
+        for (int k = 0; k < 3; ++k) { at[dir][k] = n; n += whole(sizes[k] * sizeof(int)); }
+    }
+    const size_t coef = n + whole((size_t)kChainCell * c->nCells * sizeof(double));
+    const size_t bytes = coef + whole((size_t)std::max(plans[0].slots, plans[1].slots) * kEdgeCoefs * real);
+    if (cudaMalloc((void **)&c->d_chain, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        c->d_chain = nullptr;
+        return OFG_OK;
+    }
+    for (int dir = 0; dir < 2; ++dir) {
+        const Plan &P = plans[dir];
+        const std::vector<int> *parts[3] = {&P.lev, &P.edge, &P.ref};
+        for (int k = 0; k < 3; ++k)
+            CK(cudaMemcpyAsync(c->d_chain + at[dir][k], parts[k]->data(), parts[k]->size() * sizeof(int),
+                               cudaMemcpyHostToDevice, c->stream));
+        ChainBuf &b = c->chain[dir];
+        b.lev = reinterpret_cast<int *>(c->d_chain + at[dir][0]);
+        b.edge = reinterpret_cast<int *>(c->d_chain + at[dir][1]);
+        b.ref = reinterpret_cast<int *>(c->d_chain + at[dir][2]);
+        b.nlev = int(P.lev.size() / 4); b.slots = P.slots; b.far = P.far;
+    }
+    CK(cudaStreamSynchronize(c->stream));
+    c->d_chainCell = reinterpret_cast<double *>(c->d_chain + n);
+    c->d_chainCoef = c->d_chain + coef;
     return OFG_OK;
 }
 

@@ -40,8 +40,7 @@ struct ChainPlan {
     const int4 *lev;       // per level {first position, cells, first slot, slots per cell}
     const int *order;      // [nCells] cell at each position of the level order
     const int *ref;        // [slots] ring slot of the neighbour, ~cell when it is further back, kChainNone
-    const int2 *edge;      // [slots] {face | side << 31, neighbour}; x < 0 and y < 0 on an empty slot
-    const int *cell;       // [slots]
+    const int4 *edge;      // [slots] {face | side << 31, neighbour, cell, -}; y < 0 on an empty slot
     int nlev;
     int far;               // 1: some neighbour lies further back than the ring; 2: and within a few levels
     long long slots;
@@ -65,9 +64,10 @@ __global__ void __launch_bounds__(128) k_chain_coef(KArgs<R> A, ChainPlan P, R *
         cells[(size_t)(NEQ + 1) * A.nCells + s] = 1.0 / d;
     }
     if (s >= P.slots) return;
-    const int2 e2 = __ldg(P.edge + s);
-    if (e2.y < 0) return;
-    const int c = __ldg(P.cell + s), f = nb_face(e2), nb = e2.y;
+    const int4 e4 = __ldg(P.edge + s);
+    if (e4.y < 0) return;
+    const int2 e2 = make_int2(e4.x, e4.y);
+    const int c = e4.z, f = nb_face(e2), nb = e4.y;
     R qc[REC], qn[REC], fg[FGR];
     ld8(A.qs + (size_t)c * REC, qc);
     ld8(A.qs + (size_t)nb * REC, qn);
@@ -95,7 +95,8 @@ __global__ void __launch_bounds__(128) k_chain_mat(KArgs<R> A, ChainPlan P, doub
         cells[2 * (size_t)A.nCells + s] = 1.0 / d;
     }
     if (s >= P.slots) return;
-    const int2 e2 = __ldg(P.edge + s);
+    const int4 e4 = __ldg(P.edge + s);
+    const int2 e2 = make_int2(e4.x, e4.y);
     if (e2.y >= 0) mat[s] = (nb_right(e2) ? A.matL : A.matR)[nb_face(e2)];
 }
 

@@ -12,7 +12,7 @@
 namespace ofg {
 // One chained sweep's schedule on the device (ofg_chain.cuh)
 struct ChainBuf {
-    int *lev = nullptr, *ref = nullptr, *edge = nullptr, *cell = nullptr;
+    int *lev = nullptr, *ref = nullptr, *edge = nullptr;   // into ofg_ctx::d_chain
     int nlev = 0, far = 0;
     long long slots = 0;
 };
@@ -45,6 +45,7 @@ struct ofg_ctx {
     int *d_lo_off = nullptr, *d_lol = nullptr, *d_up_off = nullptr, *d_upl = nullptr;
     int *d_lowOrder = nullptr, *d_upOrder = nullptr, *d_key = nullptr;
     ofg::ChainBuf chain[2];                                 // lower, upper (built when the chained sweeps are in use)
+    char *d_chain = nullptr;                                // their memory
     void *d_chainCoef = nullptr;                            // edge coefficients of the sweep under way
     double *d_chainCell = nullptr;                          // and its cells' values, in the sweep's order
     unsigned *chainStatus = nullptr;                        // pinned: a chained sweep's wait ran out

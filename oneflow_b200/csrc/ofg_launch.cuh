@@ -144,7 +144,7 @@ inline bool chained(const ofg_ctx *c) { return c->tune.sweep_persistent && c->ch
 inline ChainPlan chain_plan(const ofg_ctx *c, bool lower) {
     const ChainBuf &b = c->chain[lower ? 0 : 1];
     return ChainPlan{reinterpret_cast<const int4 *>(b.lev), lower ? c->d_lowOrder : c->d_upOrder, b.ref,
-                     reinterpret_cast<const int2 *>(b.edge), b.cell, b.nlev, b.far, b.slots, c->chainStatus};
+                     reinterpret_cast<const int4 *>(b.edge), b.nlev, b.far, b.slots, c->chainStatus};
 }
 
 // Whether an FP64 sweep level runs with four lanes a cell: as long as that
