@@ -521,6 +521,8 @@ void destroy_graphs(ofg_ctx *c) {
     for (int i = 0; i < 2; ++i) {
         if (c->graph[i]) { cudaGraphExecDestroy(c->graph[i]); c->graph[i] = nullptr; }
         if (c->graphT[i]) { cudaGraphDestroy(c->graphT[i]); c->graphT[i] = nullptr; }
+        for (int last = 0; last < 2; ++last)
+            if (c->graphO[last][i]) { cudaGraphExecDestroy(c->graphO[last][i]); c->graphO[last][i] = nullptr; }
     }
     c->graphGen++;
 }
@@ -578,7 +580,7 @@ void ofg_destroy(ofg_ctx *c) {
                     c->d_lowOrder, c->d_upOrder, c->d_key, c->d_fgeo, c->d_cgeo, c->d_wdist, c->d_wall, c->d_wallG,
                     c->d_fgeoD, c->d_fofs, c->d_lr, c->d_fout,
                     c->d_q[0], c->d_q[1], c->d_qs[0], c->d_qs[1], c->d_res, c->d_dq, c->d_dt, c->d_invsr, c->d_vissr, c->d_rad,
-                    c->d_bcq, c->d_partial, c->d_npart, c->d_tpart, c->d_red, c->d_redCount, c->d_stage, c->d_scal, c->d_ext, c->d_hist, c->d_gl, c->d_mm, c->d_fix,
+                    c->d_bcq, c->d_partial, c->d_npart, c->d_tpart, c->d_red, c->d_redCount, c->d_stage, c->d_scal, c->d_ext, c->d_hist, c->d_gl[0], c->d_gl[1], c->d_mm, c->d_fix,
                     c->d_nut, c->d_dnut, c->d_resT, c->d_impsrT, c->d_matL, c->d_matR, c->d_thist, c->d_gnut};
     for (void *v : ptrs) if (v) cudaFree(v);
     free_chain(c);
@@ -777,7 +779,13 @@ int ofg_upload_mesh(ofg_ctx *c, int nNodes, const double *xN, const double *yN, 
     c->histCap = 1 << 16;
     if ((rc = upload<double>(c, &c->d_hist, nullptr, (size_t)c->histCap * NEQ))) return rc;
     if ((rc = upload<int>(c, &c->d_fix, nullptr, 1 + c->fixcap))) return rc;
-    if ((rc = upload_bytes(c, &c->d_gl, nullptr, N * GLR * rs))) return rc;
+    if ((rc = upload_bytes(c, &c->d_gl[0], nullptr, N * GLR * rs))) return rc;
+    if (c->d_gl[1]) { cudaFree(c->d_gl[1]); c->d_gl[1] = nullptr; }
+    c->gl = 0;
+    if (has_turb(c) && cudaMalloc(&c->d_gl[1], N * GLR * rs) != cudaSuccess) {   // then the iterations do not overlap
+        cudaGetLastError();
+        c->d_gl[1] = nullptr;
+    }
     bool venkatGlobal = c->p.ilim == 2 && !c->p.venkat_kh3;
     if ((rc = upload_bytes(c, &c->d_mm, nullptr, venkatGlobal ? N * MMR * rs : 0))) return rc;
     CK(cudaMemset(c->d_bcq, 0, (size_t)std::max(nBFaces, 1) * NEQ * sizeof(double)));
@@ -1079,13 +1087,38 @@ int ofg_calc_boundary(ofg_ctx *c, int tid) {
 // Measured, us an iteration in one chain / with the branch: 4,096 triangles (FP64)
 // 41.4 / 35.2, 113,886 (mixed) 88.3 / 83.0, 600,000 tetrahedra (mixed, SA) 474.7 /
 // 467.0.  The CFL advance beside the gradients was not worth its fork and join.
+//
+// With an SA solver the next iteration's gradients, which read the NS state
+// alone, run beside the whole SA stage (into the other set of records: the SA
+// source reads this iteration's), and the gradient of nu~ beside the boundary
+// conditions: all wait on memory with the SMs' issue slots mostly empty.  The
+// gradients of a call's first iteration run ahead of its graph, and its last
+// iteration's graph has none.  Measured, us an iteration in one chain /
+// overlapped: 600,000 tetrahedra (mixed) 468.0 / 458.1, 769,000 cells (mixed)
+// 630.4 / 618.1, 312,500 cells (FP64) 604.6 / 568.9; at 6 million (mixed), where
+// each pass by itself keeps memory busy, 3946 / 3944.  Begun later, beside the
+// sweeps alone, the gradients gained less (FP64: 583.5).
 enum Fork { F_MAIN, F_FORK, F_SIDE, F_JOIN };   // a task of the chain; the branch's start, a task of it, its end
-struct Step { Fork where; int task; };
-static const Step kNsSteps[] = {{F_MAIN, T_GRADLIM0}, {F_MAIN, T_P_FLUX}, {F_MAIN, T_P_FSUM},
-                                {F_FORK, 0}, {F_SIDE, T_NORM}, {F_MAIN, T_CLIP0}, {F_MAIN, T_LOWER1},
-                                {F_MAIN, T_UPPER}, {F_MAIN, T_UPDATE_NEXT}, {F_MAIN, T_BOUNDARY_NEXT}};
-static const Step kTurbSteps[] = {{F_MAIN, T_TURB_RHS}, {F_FORK, 0}, {F_SIDE, T_TURB_NORM}, {F_MAIN, T_TURB_LOWER},
-                                  {F_MAIN, T_TURB_UPPER}, {F_MAIN, T_TURB_UPDATE}, {F_MAIN, T_TURB_BOUNDARY}};
+enum Stage { S_NS, S_SA, S_NEXT };              // the task's state: the iteration's, the updated one (SA; the next gradients)
+enum Need { N_ALWAYS, N_SA, N_FULL, N_MORE };   // only with an SA solver; only in a whole iteration's graph; only
+                                                // where another overlapped iteration follows
+struct Step { Fork where; int task; Stage stage; Need need; };
+static const Step kSteps[] = {
+    {F_MAIN, T_GRADLIM0, S_NS, N_FULL},
+    {F_MAIN, T_P_FLUX, S_NS, N_ALWAYS}, {F_MAIN, T_P_FSUM, S_NS, N_ALWAYS},
+    {F_FORK, 0, S_NS, N_ALWAYS}, {F_SIDE, T_NORM, S_NS, N_ALWAYS},
+    {F_MAIN, T_CLIP0, S_NS, N_ALWAYS}, {F_MAIN, T_LOWER1, S_NS, N_ALWAYS}, {F_MAIN, T_UPPER, S_NS, N_ALWAYS},
+    {F_MAIN, T_UPDATE_NEXT, S_NS, N_ALWAYS},
+    // the gradient of nu~ needs the interior of the new NS state alone
+    {F_FORK, 0, S_NS, N_SA}, {F_SIDE, T_P_TURB_GRAD, S_SA, N_SA},
+    {F_MAIN, T_BOUNDARY_NEXT, S_NS, N_ALWAYS}, {F_JOIN, 0, S_NS, N_ALWAYS},
+    {F_FORK, 0, S_NS, N_MORE}, {F_SIDE, T_GRADLIM0, S_NEXT, N_MORE},
+    {F_MAIN, T_P_TURB_FLUX, S_SA, N_SA},
+    {F_FORK, 0, S_SA, N_SA}, {F_SIDE, T_TURB_NORM, S_SA, N_SA},
+    {F_MAIN, T_TURB_LOWER, S_SA, N_SA}, {F_MAIN, T_TURB_UPPER, S_SA, N_SA}, {F_MAIN, T_TURB_UPDATE, S_SA, N_SA},
+    {F_MAIN, T_TURB_BOUNDARY, S_SA, N_SA}, {F_JOIN, 0, S_SA, N_SA}};
+
+static bool overlaps(const ofg_ctx *c) { return has_turb(c) && !multi_stage(c) && c->d_gl[1]; }
 
 static int sync_history(ofg_ctx *c) {
     size_t have = c->hist.size() / NEQ;
@@ -1123,81 +1156,100 @@ static int prepare_steps(ofg_ctx *c, int nsteps) {
     return sync(c);
 }
 
-// one outer iteration per state-buffer parity, captured once (ZERO_DQ_FIELD
-// is not needed: no kernel reads an increment it did not write this iteration)
-static int ensure_graphs(ofg_ctx *c) {
-    if (c->graph[0]) return OFG_OK;
-    int rc, saveCur = c->cur;
-    if (!c->sideStream) {
-        CK(cudaStreamCreateWithFlags(&c->sideStream, cudaStreamNonBlocking));
-        for (cudaEvent_t &e : c->forkEvent) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
-    for (int g = 0; g < 2; ++g) {
-        long long before = c->launches;
-        cudaGraph_t graph;
-        CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        c->cur = g;
-        auto run_on = [&](int t, cudaStream_t st) {
-            return c->p.precision == OFG_PREC_MIXED ? launch_task_f32(c, t, st) : launch_task_f64(c, t, st);
-        };
-        auto run = [&](int t) { return run_on(t, c->stream); };
-        auto fork = [&](cudaStream_t from, cudaStream_t to, cudaEvent_t e) {   // `to` goes on after what `from` holds
-            cudaError_t q = cudaEventRecord(e, from);
-            if (q == cudaSuccess) q = cudaStreamWaitEvent(to, e, 0);
-            return q == cudaSuccess ? OFG_OK : c->fail(OFG_E_CUDA, std::string("graph branch: ") + cudaGetErrorString(q));
-        };
-        auto step = [&](const Step &t) {
-            switch (t.where) {
-            case F_FORK: return fork(c->stream, c->sideStream, c->forkEvent[0]);
-            case F_JOIN: return fork(c->sideStream, c->stream, c->forkEvent[1]);
-            case F_SIDE: return run_on(t.task, c->sideStream);
-            default: return run(t.task);
-            }
-        };
-        if (multi_stage(c)) {
-            // TimeIntegral::RungeKutta (codes/solver/src/TimeIntegral.cpp:81-111): the
-            // time step once, then per stage the residual, CALC_LHS with
-            // lhscoef = 1/(stage+1), UPDATE_FLOWFIELD and CALC_BOUNDARY, each
-            // stage reading the buffer the previous one wrote.  (LOAD_Q copies q
-            // to a field UPDATE_FLOWFIELD never reads -- GetUpdateField,
-            // codes/update/src/Update.cpp:64-86, sets its pointer arguments by
-            // value -- so it has no effect on the iterates and is not run.)
-            const int st[] = {T_ADVANCE, T_TIMESTEP};
-            for (int t : st)
-                if ((rc = run(t))) { cudaStreamEndCapture(c->stream, &graph); c->cur = saveCur; return rc; }
-            for (int k = 0; k < c->p.rk_stage; ++k) {
-                c->cur = g ^ (k & 1);
-                c->lhsCoef = 1.0 / (k + 1);
-                const int stage[] = {T_RESIDUAL, T_CALC_LHS, T_UPDATE, T_BOUNDARY_NEXT};
-                for (int t : stage)
-                    if ((rc = run(t))) { cudaStreamEndCapture(c->stream, &graph); c->cur = saveCur; return rc; }
-            }
-            if ((rc = run(T_NORM))) { cudaStreamEndCapture(c->stream, &graph); c->cur = saveCur; return rc; }
-        } else {
-            for (const Step &t : kNsSteps)
-                if ((rc = step(t))) { cudaStreamEndCapture(c->stream, &graph); c->cur = saveCur; return rc; }
-            c->cur = g ^ 1;
-            if (has_turb(c))
-                for (const Step &t : kTurbSteps)
-                    if ((rc = step(t))) { cudaStreamEndCapture(c->stream, &graph); c->cur = saveCur; return rc; }
-            if ((rc = step({F_JOIN, 0}))) { cudaStreamEndCapture(c->stream, &graph); c->cur = saveCur; return rc; }
+enum GraphKind { G_WHOLE, G_MORE, G_LAST };   // an iteration by itself; an overlapped one with another after it; the last
+
+// one outer iteration from parity g, captured (ZERO_DQ_FIELD is not needed: no
+// kernel reads an increment it did not write this iteration)
+static int capture_iteration(ofg_ctx *c, int g, GraphKind kind, cudaGraph_t *out, cudaGraphExec_t *exec, long long *kernels) {
+    int rc = OFG_OK;
+    const int saveCur = c->cur, saveGl = c->gl;
+    const long long before = c->launches;
+    cudaGraph_t graph = nullptr;
+    CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+    c->cur = g;
+    c->gl = kind == G_WHOLE ? 0 : g;
+    auto run_on = [&](int t, cudaStream_t st) {
+        return c->p.precision == OFG_PREC_MIXED ? launch_task_f32(c, t, st) : launch_task_f64(c, t, st);
+    };
+    auto fork = [&](cudaStream_t from, cudaStream_t to, cudaEvent_t e) {   // `to` goes on after what `from` holds
+        cudaError_t q = cudaEventRecord(e, from);
+        if (q == cudaSuccess) q = cudaStreamWaitEvent(to, e, 0);
+        return q == cudaSuccess ? OFG_OK : c->fail(OFG_E_CUDA, std::string("graph branch: ") + cudaGetErrorString(q));
+    };
+    if (multi_stage(c)) {
+        // TimeIntegral::RungeKutta (codes/solver/src/TimeIntegral.cpp:81-111): the
+        // time step once, then per stage the residual, CALC_LHS with
+        // lhscoef = 1/(stage+1), UPDATE_FLOWFIELD and CALC_BOUNDARY, each
+        // stage reading the buffer the previous one wrote.  (LOAD_Q copies q
+        // to a field UPDATE_FLOWFIELD never reads -- GetUpdateField,
+        // codes/update/src/Update.cpp:64-86, sets its pointer arguments by
+        // value -- so it has no effect on the iterates and is not run.)
+        for (int t : {T_ADVANCE, T_TIMESTEP})
+            if (!rc) rc = run_on(t, c->stream);
+        for (int k = 0; k < c->p.rk_stage; ++k) {
+            c->cur = g ^ (k & 1);
+            c->lhsCoef = 1.0 / (k + 1);
+            for (int t : {T_RESIDUAL, T_CALC_LHS, T_UPDATE, T_BOUNDARY_NEXT})
+                if (!rc) rc = run_on(t, c->stream);
         }
-        CK(cudaStreamEndCapture(c->stream, &graph));
-        CK(cudaGraphInstantiate(&c->graph[g], graph, 0));
-        c->graphT[g] = graph;   // kept: a batch embeds it as a child graph
-        c->graphKernels[g] = c->launches - before;
-        c->launches = before;
+        if (!rc) rc = run_on(T_NORM, c->stream);
+    } else {
+        for (const Step &t : kSteps) {
+            if (rc) break;
+            if ((t.need == N_SA && !has_turb(c)) || (t.need == N_FULL && kind != G_WHOLE) ||
+                (t.need == N_MORE && kind != G_MORE))
+                continue;
+            c->cur = t.stage == S_NS ? g : g ^ 1;
+            if (kind != G_WHOLE) c->gl = t.stage == S_NEXT ? g ^ 1 : g;
+            switch (t.where) {
+            case F_FORK: rc = fork(c->stream, c->sideStream, c->forkEvent[0]); break;
+            case F_JOIN: rc = fork(c->sideStream, c->stream, c->forkEvent[1]); break;
+            case F_SIDE: rc = run_on(t.task, c->sideStream); break;
+            default: rc = run_on(t.task, c->stream); break;
+            }
+        }
     }
     c->cur = saveCur;
+    c->gl = saveGl;
+    *kernels = c->launches - before;
+    c->launches = before;
+    cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
+    if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(exec, graph, 0);
+    if (!rc && e != cudaSuccess) rc = c->fail(OFG_E_CUDA, std::string("iteration graph: ") + cudaGetErrorString(e));
+    if (!rc && out) *out = graph;
+    else if (graph) cudaGraphDestroy(graph);
+    return rc;
+}
+
+// the graphs of whole iterations, or of overlapped ones
+static int ensure_graphs(ofg_ctx *c, bool whole = true) {
+    if (whole ? c->graph[1] != nullptr : c->graphO[1][1] != nullptr) return OFG_OK;
+    if (!c->sideStream) {
+        int least = 0, greatest = 0;   // the branch gives way to the chain
+        CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        CK(cudaStreamCreateWithPriority(&c->sideStream, cudaStreamNonBlocking, least));
+        for (cudaEvent_t &e : c->forkEvent) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    int rc;
+    for (int g = 0; g < 2; ++g) {
+        if (whole) {   // the templates are kept: a batch embeds them as child graphs
+            if ((rc = capture_iteration(c, g, G_WHOLE, &c->graphT[g], &c->graph[g], &c->graphKernels[g]))) return rc;
+            continue;
+        }
+        for (int last = 0; last < 2; ++last)
+            if ((rc = capture_iteration(c, g, last ? G_LAST : G_MORE, nullptr, &c->graphO[last][g], &c->graphOKernels[last][g])))
+                return rc;
+    }
     return OFG_OK;
 }
 
 // host bookkeeping of one outer iteration launched from parity c->cur (the
 // multi-stage scheme moves between the two state buffers once per stage)
-static void account_step(ofg_ctx *c) {
-    c->launches += c->graphKernels[c->cur];
+static void account_step(ofg_ctx *c, bool overlapped = false, bool last = false) {
+    c->launches += overlapped ? c->graphOKernels[last][c->cur] : c->graphKernels[c->cur];
     int flips = multi_stage(c) ? c->p.rk_stage : 1;
     c->lastResBuf = c->cur ^ ((flips - 1) & 1);   // the buffer the last residual pass read
+    c->gl = overlapped ? c->lastResBuf : 0;
     c->cur ^= flips & 1;
     c->outerSteps++;
 }
@@ -1205,10 +1257,16 @@ static void account_step(ofg_ctx *c) {
 int ofg_step(ofg_ctx *c, int nsteps) {
     int rc = prepare_steps(c, nsteps);
     if (rc) return rc;
-    if ((rc = ensure_graphs(c))) return rc;
+    const bool overlap = overlaps(c) && nsteps > 0;
+    if ((rc = ensure_graphs(c, !overlap))) return rc;
+    if (overlap) {   // the first iteration's gradients
+        c->gl = c->cur;
+        if ((rc = launch(c, T_GRADLIM0))) return rc;
+    }
     for (int it = 0; it < nsteps; ++it) {
-        CK(cudaGraphLaunch(c->graph[c->cur], c->stream));
-        account_step(c);
+        const bool last = it + 1 == nsteps;
+        CK(cudaGraphLaunch(overlap ? c->graphO[last][c->cur] : c->graph[c->cur], c->stream));
+        account_step(c, overlap, last);
     }
     if ((rc = sync(c))) return rc;
     return sync_history(c);
@@ -1414,7 +1472,7 @@ int ofg_forces(ofg_ctx *c, double aref, double *out) {
             // (still in the other buffer), or none before any pass
             if (c->lastResBuf < 0) {
                 size_t rs = c->p.precision == OFG_PREC_MIXED ? sizeof(float) : sizeof(double);
-                CK(cudaMemsetAsync(c->d_gl, 0, (size_t)c->nCells * GLR * rs, c->stream));
+                CK(cudaMemsetAsync(c->d_gl[c->gl], 0, (size_t)c->nCells * GLR * rs, c->stream));
             } else {
                 int save = c->cur;
                 c->cur = c->lastResBuf;
@@ -1466,11 +1524,11 @@ int ofg_download_field(ofg_ctx *c, int tid, const char *name, double *out, int64
         buf.assign((size_t)NEQ * nT, 0.0);
         if (c->p.precision == OFG_PREC_MIXED) {
             std::vector<float> tmp((size_t)N * GLR);
-            cudaMemcpy(tmp.data(), c->d_gl, tmp.size() * sizeof(float), cudaMemcpyDeviceToHost);
+            cudaMemcpy(tmp.data(), c->d_gl[c->gl], tmp.size() * sizeof(float), cudaMemcpyDeviceToHost);
             for (int e = 0; e < NEQ; ++e) for (int64_t i = 0; i < N; ++i) buf[(size_t)e * nT + i] = tmp[(size_t)i * GLR + off + e * step];
         } else {
             std::vector<double> tmp((size_t)N * GLR);
-            cudaMemcpy(tmp.data(), c->d_gl, tmp.size() * sizeof(double), cudaMemcpyDeviceToHost);
+            cudaMemcpy(tmp.data(), c->d_gl[c->gl], tmp.size() * sizeof(double), cudaMemcpyDeviceToHost);
             for (int e = 0; e < NEQ; ++e) for (int64_t i = 0; i < N; ++i) buf[(size_t)e * nT + i] = tmp[(size_t)i * GLR + off + e * step];
         }
     };

@@ -74,7 +74,9 @@ struct ofg_ctx {
     double *d_npart = nullptr, *d_tpart = nullptr;          // per-block sums of squares of the residuals
     double *d_red = nullptr;                                // [kRedBlocks][5] block sums of the grid reductions
     unsigned int *d_redCount = nullptr;                     // their ticket counter (0 between launches)
-    void *d_gl = nullptr, *d_mm = nullptr;                  // gradient+limiter records, min/max differences
+    void *d_gl[2] = {nullptr, nullptr};                     // gradient+limiter records; a second set for the overlapped iteration
+    int gl = 0;                                             // the set in use: the last residual pass's
+    void *d_mm = nullptr;                                   // min/max differences
     int *d_fix = nullptr;
     // SA solver
     double *d_nut = nullptr, *d_dnut = nullptr, *d_resT = nullptr, *d_impsrT = nullptr, *d_matL = nullptr,
@@ -93,6 +95,8 @@ struct ofg_ctx {
     cudaGraph_t graphT[2] = {nullptr, nullptr};   // their templates (child graphs of a batch)
     unsigned graphGen = 0;                         // bumped whenever the graphs are dropped
     long long graphKernels[2] = {0, 0};
+    cudaGraphExec_t graphO[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};   // overlapped iterations: [last of a call][parity]
+    long long graphOKernels[2][2] = {{0, 0}, {0, 0}};
 
     int fail(int code, const std::string &msg) {
         err = msg;

@@ -53,7 +53,7 @@ KArgs<R> make_args(ofg_ctx *c, bool onCurrent) {
     }
     A.res = c->d_res; A.dq = static_cast<R *>(c->d_dq); A.dt = c->d_dt; A.invsr = c->d_invsr; A.vissr = c->d_vissr;
     A.rad = c->d_rad;
-    A.bcq = c->d_bcq; A.gl = static_cast<R *>(c->d_gl); A.mm = static_cast<R *>(c->d_mm);
+    A.bcq = c->d_bcq; A.gl = static_cast<R *>(c->d_gl[c->gl]); A.mm = static_cast<R *>(c->d_mm);
     A.scal = c->d_scal; A.ext = c->d_ext; A.fixlist = c->d_fix; A.fixcap = c->fixcap;
     A.npart = c->d_npart; A.tpart = c->d_tpart; A.red = c->d_red; A.redCount = c->d_redCount;
     A.nut = c->d_nut; A.dnut = c->d_dnut; A.resT = c->d_resT; A.impsrT = c->d_impsrT;

@@ -19,23 +19,12 @@ __device__ __forceinline__ double sa_vist(const DevParams &P, double rho, double
     return fmin(vl * P.max_vis_ratio, v);
 }
 
-// write the eddy viscosity of cell i into the master record and its FP32
-// copy, rewriting whole 32-byte sectors (p T mu_l mu_t of the master, the
-// whole copy) rather than single words
+// write the eddy viscosity of cell i into the master record and its FP32 copy:
+// that word alone, a gradient pass running beside the SA stage reads the others
 template <typename R>
 __device__ __forceinline__ void put_vist(const KArgs<R> &A, int i, double v) {
-    double2 *m = reinterpret_cast<double2 *>(const_cast<double *>(A.q) + (size_t)i * REC);
-    double2 a = m[2], b = m[3];
-    b.y = v;
-    m[2] = a;
-    m[3] = b;
-    if (sizeof(R) == 4) {
-        float4 *s = reinterpret_cast<float4 *>(const_cast<R *>(A.qs) + (size_t)i * REC);
-        float4 s0 = s[0], s1 = s[1];
-        s1.w = float(v);
-        s[0] = s0;
-        s[1] = s1;
-    }
+    const_cast<double *>(A.q)[(size_t)i * REC + IMT] = v;
+    if (sizeof(R) == 4) const_cast<R *>(A.qs)[(size_t)i * REC + IMT] = R(v);
 }
 
 // TurbBcSolver face rules (codes/turb/src/TurbBcSolver.cpp:51-262); the

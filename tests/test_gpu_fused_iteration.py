@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from oneflow_b200 import meshgen, params as P
-from oneflow_b200.solver import LUSGS_SEQUENCE, NS_SOLVER, TURB_SOLVER, Solver
+from oneflow_b200.solver import LUSGS_SEQUENCE, NS_SOLVER, TURB_SOLVER, Batch, Solver
 from oneflow_b200.walldist import plate_wall_distance
 
 pytestmark = pytest.mark.gpu
@@ -49,3 +49,26 @@ def test_fused_iterations_are_the_tasks(name):
     assert np.array_equal(a.res_history(), np.array(norms))
     if prm.vismodel >= 3:
         assert np.array_equal(a.state(TURB_SOLVER), b.state(TURB_SOLVER))
+
+
+@pytest.mark.parametrize("name", ["plate3d", "plate3d_fp64"])
+def test_overlapped_iterations_are_the_whole_ones(name):
+    """ofg_step runs the next gradients beside the SA stage; a batch runs whole
+    iterations.  State, forces and the gradient records agree bit for bit after
+    calls of one, two and three iterations, and when the two alternate."""
+    m, prm = case(name)
+    a, b = Solver(m, prm), Solver(m, prm)
+    a.init_flowfield()
+    b.init_flowfield()
+    batch, own = Batch([b]), Batch([a])
+    for n, whole in ((1, False), (2, False), (3, False), (1, True), (2, False)):
+        (own if whole else a).step(n)
+        batch.step(n)
+        assert np.array_equal(a.state(), b.state())
+        assert np.array_equal(a.state(TURB_SOLVER), b.state(TURB_SOLVER))
+        assert np.array_equal(a.forces(), b.forces())
+        for field in ("dqdx", "dqdz", "limiter"):
+            assert np.array_equal(a.field(field), b.field(field))
+    assert np.array_equal(a.res_history(), b.res_history())
+    batch.close()
+    own.close()
