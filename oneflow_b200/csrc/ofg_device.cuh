@@ -8,6 +8,7 @@
 // from the FP64 state records, so that the FP32 rounding of the large
 // low-Mach pressure and enthalpy terms sets no floor under the residual).
 #pragma once
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 

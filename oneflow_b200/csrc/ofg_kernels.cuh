@@ -824,48 +824,56 @@ __device__ __forceinline__ void face_vis_flux(const DevParams &P, const R *ql, c
     face_vis_flux<R, VV>(P, ql, qr, dlr, fg, cgl, cgr, gl, gr, bface, fv);
 }
 
-// The end of the residual pass of one cell: its residual and block sums of
-// squares (for the norms), and the local time step from the summed face
-// radii (UTimeStep::CalcInvTimeStep / CalcVisTimeStep) with the zone-wide
-// minimum.  The block epilogue sums the squares in a fixed order
-// (deterministic) and lowers the minimum time step by an atomic minimum on
-// the bit pattern (non-negative doubles order like their bits).  Every thread
-// of the block calls it; `active` is false past the last cell.
+// The end of the residual pass of one cell: its residual, whose squares it
+// leaves in sq, and the local time step from the summed face radii
+// (UTimeStep::CalcInvTimeStep / CalcVisTimeStep), which it returns
+template <bool doRes, bool doDt>
+__device__ __forceinline__ double residual_cell(const DevParams &P, double *res, double *dt, double *invsr,
+                                                double *vissr, const double *scal, int c, const double *acc, double inv,
+                                                double vis, double vol, double *sq) {
+    if (doRes) {
+        double *o = res + (size_t)c * NEQ;
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) { o[e] = acc[e]; sq[e] = acc[e] * acc[e]; }
+    }
+    if (!doDt) return 1.0e40;
+    double cfl = scal[S_CFL];
+    double ts;
+    if (P.timestepModel == 1) {
+        ts = P.global_dt;
+    } else {
+        ts = cfl * vol / inv;
+        if (P.vismodel > 0 && P.visTimeStepModel > 0) {
+            double vts = cfl * vol / vis;
+            ts *= vts / (ts + vts);
+        }
+    }
+    invsr[c] = inv;
+    vissr[c] = vis;
+    dt[c] = ts;
+    return ts;
+}
+
+// the zone-wide minimum of the time step, by an atomic minimum on the bit
+// pattern (non-negative doubles order like their bits)
+__device__ __forceinline__ void lower_min_dt(double *scal, double m) {
+    atomicMin(reinterpret_cast<unsigned long long *>(scal + S_MINDT), (unsigned long long)__double_as_longlong(m));
+}
+
+// residual_cell and the block's sums of squares (for the norms), added in a
+// fixed order (deterministic), and its least time step.  Every thread of the
+// block calls it; `active` is false past the last cell.
 template <bool doRes, bool doDt>
 __device__ __forceinline__ void residual_epilogue(const DevParams &P, double *res, double *dt, double *invsr,
                                                   double *vissr, double *npart, double *scal, int c, bool active,
                                                   const double *acc, double inv, double vis, double vol) {
     double mydt = 1.0e40;
     double sq[NEQ] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    if (active) {
-        if (doRes) {
-            double *o = res + (size_t)c * NEQ;
-#pragma unroll
-            for (int e = 0; e < NEQ; ++e) { o[e] = acc[e]; sq[e] = acc[e] * acc[e]; }
-        }
-        if (doDt) {
-            double cfl = scal[S_CFL];
-            double ts;
-            if (P.timestepModel == 1) {
-                ts = P.global_dt;
-            } else {
-                ts = cfl * vol / inv;
-                if (P.vismodel > 0 && P.visTimeStepModel > 0) {
-                    double vts = cfl * vol / vis;
-                    ts *= vts / (ts + vts);
-                }
-            }
-            invsr[c] = inv;
-            vissr[c] = vis;
-            dt[c] = ts;
-            mydt = ts;
-        }
-    }
+    if (active) mydt = residual_cell<doRes, doDt>(P, res, dt, invsr, vissr, scal, c, acc, inv, vis, vol, sq);
     if (doRes) block_sum_to<NEQ>(sq, npart + (size_t)blockIdx.x * NEQ);
     if (doDt) {
         double m = block_min(mydt);
-        if (threadIdx.x == 0)
-            atomicMin(reinterpret_cast<unsigned long long *>(scal + S_MINDT), (unsigned long long)__double_as_longlong(m));
+        if (threadIdx.x == 0) lower_min_dt(scal, m);
     }
 }
 
@@ -964,6 +972,132 @@ __global__ void __launch_bounds__(128, MinBlocks<R>::res) k_residual(KArgs<R> A)
     }
     residual_epilogue<doRes, doDt>(A.P, A.res, A.dt, A.invsr, A.vissr, A.npart, A.scal, c, active, acc, inv, vis,
                                    vol);
+}
+
+// The same with four lanes a cell, for meshes whose cells leave the SMs idle:
+// the serial chain of a cell's faces (roots and quotients at FP64 latency) is
+// then one face long.  A lane forms its face's flux in shared memory, and each
+// adds two of the seven sums over the faces in list order, so every sum has the
+// bits of k_residual's; the four blocks of a cluster hold the 128 cells of one
+// of its blocks and add their squares in its order.  Measured, us (with the
+// profile's events): 4,096 triangles (Euler, Roe) 12.5 with a thread a cell, 10.5
+// so; 8,000 quadrilaterals (laminar, SLAU2) 19.5, 15.3.  quad_residual has where
+// it pays: with more blocks than run at once its idle fourth lane and its
+// smaller blocks cost more than the chain.
+template <typename R, int MODE>
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(128) k_residual_quad(KArgs<R> A) {
+    static_assert(sizeof(R) == 8, "the mixed path runs k_face_pass + k_face_sum");
+    constexpr bool doRes = MODE != 1, doDt = MODE != 2;
+    constexpr int NV = NEQ + 2;   // flux, inviscid and viscous radius
+    __shared__ double sFace[4][32][NV], sSq[32][NEQ], sDt[32], sPart[4][NEQ];
+    const auto cluster = cooperative_groups::this_cluster();
+    if (doRes) cluster.barrier_arrive();   // this block runs: its sPart may be written
+    const DevParams &P = A.P;
+    const int c = blockIdx.x * 32 + (threadIdx.x >> 2), j = threadIdx.x & 3;
+    const bool active = c < A.nCells;
+    // a lane's sums: value j, and value j + 4 (lane 0: the fifth flux, lanes 1
+    // and 2 the radii).  LoadResiduals: res = -rhs, rhs = 0
+    double acc0 = -0.0, acc1 = j == 0 ? -0.0 : 0.0;
+    double (*face)[NV] = sFace[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, quad = lane & ~3;
+    R qc[REC], cgc[CGR] = {}, glc[GLR];
+    const bool needGl = doRes && (P.ilim != -1 || P.vismodel > 0);
+    int b = 0, en = 0;
+    if (active) {
+        ld8(A.qs + (size_t)c * REC, qc);
+        ld4(A.cgeo + (size_t)c * CGR, cgc);
+        if (needGl) ld_gl(A.gl + (size_t)c * GLR, glc);
+        b = A.nb_off[c];
+        en = A.nb_off[c + 1];
+    }
+    const R gam = R(P.gama), ce1 = R(P.centropy1), ce2 = R(P.centropy2), orey = R(P.oreynolds);
+    // the inviscid faces, then the viscous ones, as k_residual adds them
+    for (int pass = 0; pass < (doRes && P.vismodel > 0 ? 2 : 1); ++pass) {
+        for (int k0 = b; __any_sync(0xffffffffu, k0 < en); k0 += 4) {
+            if (k0 + j < en) {
+                double si = 0.0, sv = 0.0;
+                const int2 e2 = __ldg(&A.nbl[k0 + j]);
+                const int f = nb_face(e2), nb = e2.y;
+                const bool right = nb_right(e2);
+                R qn[REC], cgn[CGR], fg[FGR], gln[GLR];
+                ld8(A.qs + (size_t)nb * REC, qn);
+                ld8(A.fgeo + (size_t)f * FGR, fg);
+                ld4(A.cgeo + (size_t)nb * CGR, cgn);
+                const bool ghost = nb >= A.nCells;
+                if (needGl && !ghost) ld_gl(A.gl + (size_t)nb * GLR, gln);
+                const R *ql = right ? qn : qc, *qr = right ? qc : qn;
+                const R *cgl = right ? cgn : cgc, *cgr = right ? cgc : cgn;
+                // ghost cells carry their interior cell's gradient (UGrad.cpp:140-148)
+                const R *gll = right ? gln : glc, *glr = (right || ghost) ? glc : gln;
+                R fl[NEQ] = {}, scale = R(0);
+                if (pass == 0) {
+                    if (doDt) {
+                        si = face_inv_spec(P, ql, qr, fg);
+                        if (P.vismodel > 0) sv = face_vis_spec(P, ql, qr, fg, cgl, cgr);
+                    }
+                    if (doRes) {
+                        R t1[NEQ], t2[NEQ];
+                        face_states(A, f, ql, qr, fg, cgl, cgr, gll, glr, t1, t2);
+                        if (P.ischeme == 12) slau2Flux(t1, t2, fg[0], fg[1], fg[2], gam, fl);
+                        else roeFlux(t1, t2, fg[0], fg[1], fg[2], gam, P.ieigenfix, ce1, ce2, fl);
+                        scale = fg[3];
+                    }
+                } else {
+                    face_vis_flux<R, false>(P, ql, qr, fg, cgl, cgr, gll, glr, ghost, fl);
+                    scale = -orey * fg[3];
+                }
+#pragma unroll
+                for (int e = 0; e < NEQ; ++e) {
+                    const double w = double(scale * fl[e]);
+                    face[lane][e] = right ? w : -w;
+                }
+                face[lane][NEQ] = si;
+                face[lane][NEQ + 1] = sv;
+            }
+            __syncwarp();
+            for (int q = 0; q < 4 && k0 + q < en; ++q) {
+                if (doRes) acc0 += face[quad + q][j];
+                if (j < 3 && (j == 0 ? doRes : doDt && pass == 0)) acc1 += face[quad + q][j + 4];
+            }
+            __syncwarp();
+        }
+    }
+    face[lane][0] = acc0;
+    face[lane][1] = acc1;
+    __syncwarp();
+    if (j == 0) {
+        const double acc[NEQ] = {acc0, face[lane + 1][0], face[lane + 2][0], face[lane + 3][0], acc1};
+        double sq[NEQ] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        const int s = threadIdx.x >> 2;
+        sDt[s] = active ? residual_cell<doRes, doDt>(P, A.res, A.dt, A.invsr, A.vissr, A.scal, c, acc, face[lane + 1][1],
+                                                     face[lane + 2][1], double(cgc[3]), sq)
+                        : 1.0e40;
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) sSq[s][e] = sq[e];
+    }
+    __syncthreads();
+    if (doRes) cluster.barrier_wait();
+    if (threadIdx.x < 32) {   // block_sum_to's sum over a warp of cells
+        double m = sDt[threadIdx.x];
+        if (doDt) {
+            for (int o = 16; o > 0; o >>= 1) m = fmin(m, __shfl_down_sync(0xffffffffu, m, o));
+            if (threadIdx.x == 0) lower_min_dt(A.scal, m);
+        }
+        if (doRes) {
+            double *part = cluster.map_shared_rank(&sPart[0][0], 0) + cluster.block_rank() * NEQ;
+#pragma unroll
+            for (int e = 0; e < NEQ; ++e) {
+                double x = sSq[threadIdx.x][e];
+                for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+                if (threadIdx.x == 0) part[e] = x;
+            }
+        }
+    }
+    if (!doRes) return;
+    cluster.sync();
+    if (cluster.block_rank() == 0 && threadIdx.x < NEQ)   // and over the warps
+        A.npart[(size_t)(blockIdx.x >> 2) * NEQ + threadIdx.x] =
+            (sPart[0][threadIdx.x] + sPart[2][threadIdx.x]) + (sPart[1][threadIdx.x] + sPart[3][threadIdx.x]);
 }
 
 // ---------------------------------------------------------------------------

@@ -96,6 +96,14 @@ void launch_gradlim(ofg_ctx *c, const KArgs<R> &A, cudaStream_t s, bool started 
     if (limMode == 2) OFG_LAUNCH(k_limiter_global<R>, nblk(N, 128), 128, s, A);
 }
 
+// Whether the FP64 residual pass runs with four lanes a cell: as long as its
+// blocks (32 cells, two to an SM) all run at once.  Measured, us an iteration
+// with a thread a cell / four lanes: Euler triangles, 1,200 cells 27.5 / 27.5,
+// 6,144 31.5 / 29.6, 8,192 30.7 / 29.6, 10,240 31.7 / 35.7; laminar quadrilaterals,
+// 1,200 43.9 / 37.8, 8,000 44.2 / 40.5, 10,000 45.2 / 47.4; tetrahedra (SA), 5,880
+// 99.8 / 95.5, 8,976 99.9 / 95.8, 10,800 100.3 / 103.7.
+inline bool quad_residual(int cells) { return cells <= 9000; }
+
 // The flux / time-step pass of MODE (as k_residual): the FP64 path's
 // per-cell gather, or the mixed path's face pass followed by the per-cell sum
 // of the face results (part: 1 the first kernel only, 2 the second only, 3 both).
@@ -106,6 +114,7 @@ void launch_flux(ofg_ctx *c, const KArgs<R> &A, cudaStream_t s, int part = 3) {
     if constexpr (sizeof(R) == 8) {
         if (!(part & 1)) return;
         if (vv) OFG_LAUNCH((k_residual<R, MODE, true>), nblk(N, 128), 128, s, A);
+        else if (quad_residual(N)) OFG_LAUNCH((k_residual_quad<R, MODE>), 4 * nblk(N, 128), 128, s, A);
         else OFG_LAUNCH((k_residual<R, MODE>), nblk(N, 128), 128, s, A);
     } else {
         if (part & 1) {
