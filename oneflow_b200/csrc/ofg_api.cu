@@ -521,8 +521,7 @@ void destroy_graphs(ofg_ctx *c) {
     for (int i = 0; i < 2; ++i) {
         if (c->graph[i]) { cudaGraphExecDestroy(c->graph[i]); c->graph[i] = nullptr; }
         if (c->graphT[i]) { cudaGraphDestroy(c->graphT[i]); c->graphT[i] = nullptr; }
-        for (int last = 0; last < 2; ++last)
-            if (c->graphO[last][i]) { cudaGraphExecDestroy(c->graphO[last][i]); c->graphO[last][i] = nullptr; }
+        if (c->graphO[i]) { cudaGraphExecDestroy(c->graphO[i]); c->graphO[i] = nullptr; }
     }
     c->graphGen++;
 }
@@ -1092,8 +1091,9 @@ int ofg_calc_boundary(ofg_ctx *c, int tid) {
 // alone, run beside the whole SA stage (into the other set of records: the SA
 // source reads this iteration's), and the gradient of nu~ beside the boundary
 // conditions: all wait on memory with the SMs' issue slots mostly empty.  The
-// gradients of a call's first iteration run ahead of its graph, and its last
-// iteration's graph has none.  Measured, us an iteration in one chain /
+// gradients of a call's first iteration run ahead of its graph; its last
+// iteration has none, and is launched as it stands while the graphs run (a third
+// and fourth graph cost a new solver 0.6 ms).  Measured, us an iteration in one chain /
 // overlapped: 600,000 tetrahedra (mixed) 468.0 / 458.1, 769,000 cells (mixed)
 // 630.4 / 618.1, 312,500 cells (FP64) 604.6 / 568.9; at 6 million (mixed), where
 // each pass by itself keeps memory busy, 3946 / 3944.  Begun later, beside the
@@ -1156,16 +1156,13 @@ static int prepare_steps(ofg_ctx *c, int nsteps) {
     return sync(c);
 }
 
-enum GraphKind { G_WHOLE, G_MORE, G_LAST };   // an iteration by itself; an overlapped one with another after it; the last
+enum GraphKind { G_WHOLE, G_MORE, G_LAST };   // an iteration by itself; an overlapped one with another after it; the last (no graph)
 
-// one outer iteration from parity g, captured (ZERO_DQ_FIELD is not needed: no
-// kernel reads an increment it did not write this iteration)
-static int capture_iteration(ofg_ctx *c, int g, GraphKind kind, cudaGraph_t *out, cudaGraphExec_t *exec, long long *kernels) {
+// one outer iteration from parity g (ZERO_DQ_FIELD is not needed: no kernel
+// reads an increment it did not write this iteration)
+static int issue_iteration(ofg_ctx *c, int g, GraphKind kind) {
     int rc = OFG_OK;
     const int saveCur = c->cur, saveGl = c->gl;
-    const long long before = c->launches;
-    cudaGraph_t graph = nullptr;
-    CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     c->cur = g;
     c->gl = kind == G_WHOLE ? 0 : g;
     auto run_on = [&](int t, cudaStream_t st) {
@@ -1211,19 +1208,27 @@ static int capture_iteration(ofg_ctx *c, int g, GraphKind kind, cudaGraph_t *out
     }
     c->cur = saveCur;
     c->gl = saveGl;
+    return rc;
+}
+
+static int capture_iteration(ofg_ctx *c, int g, GraphKind kind, cudaGraph_t *out, long long *kernels) {
+    const long long before = c->launches;
+    cudaGraph_t graph = nullptr;
+    CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+    int rc = issue_iteration(c, g, kind);
     *kernels = c->launches - before;
     c->launches = before;
     cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
-    if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(exec, graph, 0);
     if (!rc && e != cudaSuccess) rc = c->fail(OFG_E_CUDA, std::string("iteration graph: ") + cudaGetErrorString(e));
-    if (!rc && out) *out = graph;
+    if (!rc) *out = graph;
     else if (graph) cudaGraphDestroy(graph);
     return rc;
 }
 
-// the graphs of whole iterations, or of overlapped ones
-static int ensure_graphs(ofg_ctx *c, bool whole = true) {
-    if (whole ? c->graph[1] != nullptr : c->graphO[1][1] != nullptr) return OFG_OK;
+// the graphs of overlapped iterations (G_MORE), or the templates of whole ones
+// (a batch embeds them as child graphs) and, for a context's own steps, their
+// executables (without them the first 15 iterations of 8 airfoils take 13.4 ms, with them 16.3)
+static int ensure_graphs(ofg_ctx *c, GraphKind kind, bool own) {
     if (!c->sideStream) {
         int least = 0, greatest = 0;   // the branch gives way to the chain
         CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
@@ -1232,24 +1237,28 @@ static int ensure_graphs(ofg_ctx *c, bool whole = true) {
     }
     int rc;
     for (int g = 0; g < 2; ++g) {
-        if (whole) {   // the templates are kept: a batch embeds them as child graphs
-            if ((rc = capture_iteration(c, g, G_WHOLE, &c->graphT[g], &c->graph[g], &c->graphKernels[g]))) return rc;
+        if (kind == G_MORE) {
+            if (c->graphO[g]) continue;
+            cudaGraph_t graph;
+            if ((rc = capture_iteration(c, g, kind, &graph, &c->graphOKernels[g]))) return rc;
+            cudaError_t e = cudaGraphInstantiate(&c->graphO[g], graph, 0);
+            cudaGraphDestroy(graph);
+            CK(e);
             continue;
         }
-        for (int last = 0; last < 2; ++last)
-            if ((rc = capture_iteration(c, g, last ? G_LAST : G_MORE, nullptr, &c->graphO[last][g], &c->graphOKernels[last][g])))
-                return rc;
+        if (!c->graphT[g] && (rc = capture_iteration(c, g, kind, &c->graphT[g], &c->graphKernels[g]))) return rc;
+        if (own && !c->graph[g]) CK(cudaGraphInstantiate(&c->graph[g], c->graphT[g], 0));
     }
     return OFG_OK;
 }
 
 // host bookkeeping of one outer iteration launched from parity c->cur (the
 // multi-stage scheme moves between the two state buffers once per stage)
-static void account_step(ofg_ctx *c, bool overlapped = false, bool last = false) {
-    c->launches += overlapped ? c->graphOKernels[last][c->cur] : c->graphKernels[c->cur];
+static void account_step(ofg_ctx *c, GraphKind kind = G_WHOLE) {
+    if (kind != G_LAST) c->launches += kind == G_MORE ? c->graphOKernels[c->cur] : c->graphKernels[c->cur];
     int flips = multi_stage(c) ? c->p.rk_stage : 1;
     c->lastResBuf = c->cur ^ ((flips - 1) & 1);   // the buffer the last residual pass read
-    c->gl = overlapped ? c->lastResBuf : 0;
+    c->gl = kind == G_WHOLE ? 0 : c->lastResBuf;
     c->cur ^= flips & 1;
     c->outerSteps++;
 }
@@ -1257,16 +1266,17 @@ static void account_step(ofg_ctx *c, bool overlapped = false, bool last = false)
 int ofg_step(ofg_ctx *c, int nsteps) {
     int rc = prepare_steps(c, nsteps);
     if (rc) return rc;
-    const bool overlap = overlaps(c) && nsteps > 0;
-    if ((rc = ensure_graphs(c, !overlap))) return rc;
+    const bool overlap = overlaps(c) && nsteps > 1;
+    if ((rc = ensure_graphs(c, overlap ? G_MORE : G_WHOLE, true))) return rc;
     if (overlap) {   // the first iteration's gradients
         c->gl = c->cur;
         if ((rc = launch(c, T_GRADLIM0))) return rc;
     }
     for (int it = 0; it < nsteps; ++it) {
-        const bool last = it + 1 == nsteps;
-        CK(cudaGraphLaunch(overlap ? c->graphO[last][c->cur] : c->graph[c->cur], c->stream));
-        account_step(c, overlap, last);
+        const GraphKind kind = !overlap ? G_WHOLE : it + 1 < nsteps ? G_MORE : G_LAST;
+        if (kind != G_LAST) CK(cudaGraphLaunch(kind == G_MORE ? c->graphO[c->cur] : c->graph[c->cur], c->stream));
+        else if ((rc = issue_iteration(c, c->cur, kind))) return rc;
+        account_step(c, kind);
     }
     if ((rc = sync(c))) return rc;
     return sync_history(c);
@@ -1337,7 +1347,7 @@ int ofg_batch_step(ofg_batch *b, int nsteps) {
     for (int i = 0; i < n; ++i) {
         ofg_ctx *c = b->ctx[i];
         int rc = prepare_steps(c, nsteps);
-        if (!rc) rc = ensure_graphs(c);
+        if (!rc) rc = ensure_graphs(c, G_WHOLE, false);
         if (rc) return b->fail(rc, "context " + std::to_string(i) + ": " + c->err);
     }
     // the two batch graphs stay valid while every context keeps the graphs

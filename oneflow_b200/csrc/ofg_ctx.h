@@ -95,8 +95,8 @@ struct ofg_ctx {
     cudaGraph_t graphT[2] = {nullptr, nullptr};   // their templates (child graphs of a batch)
     unsigned graphGen = 0;                         // bumped whenever the graphs are dropped
     long long graphKernels[2] = {0, 0};
-    cudaGraphExec_t graphO[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};   // overlapped iterations: [last of a call][parity]
-    long long graphOKernels[2][2] = {{0, 0}, {0, 0}};
+    cudaGraphExec_t graphO[2] = {nullptr, nullptr};   // iterations that the next one's gradients overlap
+    long long graphOKernels[2] = {0, 0};
 
     int fail(int code, const std::string &msg) {
         err = msg;
