@@ -1156,7 +1156,8 @@ static int prepare_steps(ofg_ctx *c, int nsteps) {
     return sync(c);
 }
 
-enum GraphKind { G_WHOLE, G_MORE, G_LAST };   // an iteration by itself; an overlapped one with another after it; the last (no graph)
+enum GraphKind { G_WHOLE, G_BATCH, G_MORE, G_LAST };   // an iteration by itself; a batch member's; an overlapped one with another
+                                                       // after it; the last (no graph)
 
 // one outer iteration from parity g (ZERO_DQ_FIELD is not needed: no kernel
 // reads an increment it did not write this iteration)
@@ -1164,7 +1165,9 @@ static int issue_iteration(ofg_ctx *c, int g, GraphKind kind) {
     int rc = OFG_OK;
     const int saveCur = c->cur, saveGl = c->gl;
     c->cur = g;
-    c->gl = kind == G_WHOLE ? 0 : g;
+    c->gl = kind <= G_BATCH ? 0 : g;
+    // a batch's members fill the GPU side by side: one plain chain each, no extra lanes
+    c->crowded = kind == G_BATCH;
     auto run_on = [&](int t, cudaStream_t st) {
         return c->p.precision == OFG_PREC_MIXED ? launch_task_f32(c, t, st) : launch_task_f64(c, t, st);
     };
@@ -1193,11 +1196,15 @@ static int issue_iteration(ofg_ctx *c, int g, GraphKind kind) {
     } else {
         for (const Step &t : kSteps) {
             if (rc) break;
-            if ((t.need == N_SA && !has_turb(c)) || (t.need == N_FULL && kind != G_WHOLE) ||
+            if ((t.need == N_SA && !has_turb(c)) || (t.need == N_FULL && kind > G_BATCH) ||
                 (t.need == N_MORE && kind != G_MORE))
                 continue;
             c->cur = t.stage == S_NS ? g : g ^ 1;
-            if (kind != G_WHOLE) c->gl = t.stage == S_NEXT ? g ^ 1 : g;
+            if (kind > G_BATCH) c->gl = t.stage == S_NEXT ? g ^ 1 : g;
+            if (kind == G_BATCH) {
+                if (t.where == F_MAIN || t.where == F_SIDE) rc = run_on(t.task, c->stream);
+                continue;
+            }
             switch (t.where) {
             case F_FORK: rc = fork(c->stream, c->sideStream, c->forkEvent[0]); break;
             case F_JOIN: rc = fork(c->sideStream, c->stream, c->forkEvent[1]); break;
@@ -1208,6 +1215,7 @@ static int issue_iteration(ofg_ctx *c, int g, GraphKind kind) {
     }
     c->cur = saveCur;
     c->gl = saveGl;
+    c->crowded = false;
     return rc;
 }
 
@@ -1225,10 +1233,10 @@ static int capture_iteration(ofg_ctx *c, int g, GraphKind kind, cudaGraph_t *out
     return rc;
 }
 
-// the graphs of overlapped iterations (G_MORE), or the templates of whole ones
-// (a batch embeds them as child graphs) and, for a context's own steps, their
-// executables (without them the first 15 iterations of 8 airfoils take 13.4 ms, with them 16.3)
-static int ensure_graphs(ofg_ctx *c, GraphKind kind, bool own) {
+// the graphs of a context's own steps, whole (G_WHOLE) or overlapped (G_MORE), or
+// the templates that a batch embeds as child graphs (G_BATCH; without executables
+// of their own: the first 15 iterations of 8 airfoils take 13.4 ms, with them 16.3)
+static int ensure_graphs(ofg_ctx *c, GraphKind kind) {
     if (!c->sideStream) {
         int least = 0, greatest = 0;   // the branch gives way to the chain
         CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
@@ -1237,17 +1245,17 @@ static int ensure_graphs(ofg_ctx *c, GraphKind kind, bool own) {
     }
     int rc;
     for (int g = 0; g < 2; ++g) {
-        if (kind == G_MORE) {
-            if (c->graphO[g]) continue;
-            cudaGraph_t graph;
-            if ((rc = capture_iteration(c, g, kind, &graph, &c->graphOKernels[g]))) return rc;
-            cudaError_t e = cudaGraphInstantiate(&c->graphO[g], graph, 0);
-            cudaGraphDestroy(graph);
-            CK(e);
+        if (kind == G_BATCH) {
+            if (!c->graphT[g] && (rc = capture_iteration(c, g, kind, &c->graphT[g], &c->graphKernels[g]))) return rc;
             continue;
         }
-        if (!c->graphT[g] && (rc = capture_iteration(c, g, kind, &c->graphT[g], &c->graphKernels[g]))) return rc;
-        if (own && !c->graph[g]) CK(cudaGraphInstantiate(&c->graph[g], c->graphT[g], 0));
+        cudaGraphExec_t &exec = kind == G_MORE ? c->graphO[g] : c->graph[g];
+        if (exec) continue;
+        cudaGraph_t graph;
+        if ((rc = capture_iteration(c, g, kind, &graph, kind == G_MORE ? &c->graphOKernels[g] : &c->graphKernels[g]))) return rc;
+        cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
+        cudaGraphDestroy(graph);
+        CK(e);
     }
     return OFG_OK;
 }
@@ -1267,7 +1275,7 @@ int ofg_step(ofg_ctx *c, int nsteps) {
     int rc = prepare_steps(c, nsteps);
     if (rc) return rc;
     const bool overlap = overlaps(c) && nsteps > 1;
-    if ((rc = ensure_graphs(c, overlap ? G_MORE : G_WHOLE, true))) return rc;
+    if ((rc = ensure_graphs(c, overlap ? G_MORE : G_WHOLE))) return rc;
     if (overlap) {   // the first iteration's gradients
         c->gl = c->cur;
         if ((rc = launch(c, T_GRADLIM0))) return rc;
@@ -1347,7 +1355,7 @@ int ofg_batch_step(ofg_batch *b, int nsteps) {
     for (int i = 0; i < n; ++i) {
         ofg_ctx *c = b->ctx[i];
         int rc = prepare_steps(c, nsteps);
-        if (!rc) rc = ensure_graphs(c, G_WHOLE, false);
+        if (!rc) rc = ensure_graphs(c, G_BATCH);
         if (rc) return b->fail(rc, "context " + std::to_string(i) + ": " + c->err);
     }
     // the two batch graphs stay valid while every context keeps the graphs

@@ -97,6 +97,7 @@ struct ofg_ctx {
     long long graphKernels[2] = {0, 0};
     cudaGraphExec_t graphO[2] = {nullptr, nullptr};   // iterations that the next one's gradients overlap
     long long graphOKernels[2] = {0, 0};
+    bool crowded = false;   // launching for a batch: other members keep the GPU busy
 
     int fail(int code, const std::string &msg) {
         err = msg;

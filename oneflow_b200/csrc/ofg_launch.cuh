@@ -114,7 +114,7 @@ void launch_flux(ofg_ctx *c, const KArgs<R> &A, cudaStream_t s, int part = 3) {
     if constexpr (sizeof(R) == 8) {
         if (!(part & 1)) return;
         if (vv) OFG_LAUNCH((k_residual<R, MODE, true>), nblk(N, 128), 128, s, A);
-        else if (quad_residual(N)) OFG_LAUNCH((k_residual_quad<R, MODE>), 4 * nblk(N, 128), 128, s, A);
+        else if (!c->crowded && quad_residual(N)) OFG_LAUNCH((k_residual_quad<R, MODE>), 4 * nblk(N, 128), 128, s, A);
         else OFG_LAUNCH((k_residual<R, MODE>), nblk(N, 128), 128, s, A);
     } else {
         if (part & 1) {
@@ -281,7 +281,7 @@ int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
                 default: OFG_LAUNCH((k_lusgs_lower<R, 8>), nblk(cnt, bs), bs, s, A, ord, st, cnt); break;
                 }
             } else {
-                if (quad_level(cnt)) OFG_LAUNCH((k_lusgs_quad<R, true>), nblk(4LL * cnt, 128), 128, s, A, ord, st, cnt);
+                if (!c->crowded && quad_level(cnt)) OFG_LAUNCH((k_lusgs_quad<R, true>), nblk(4LL * cnt, 128), 128, s, A, ord, st, cnt);
                 else OFG_LAUNCH(k_lusgs_lower<R>, nblk(cnt, 128), 128, s, A, ord, st, cnt);
             }
         }
@@ -305,7 +305,7 @@ int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
                 default: OFG_LAUNCH((k_lusgs_upper<R, 8>), nblk(cnt, bs), bs, s, A, ord, st, cnt); break;
                 }
             } else {
-                if (quad_level(cnt)) OFG_LAUNCH((k_lusgs_quad<R, false>), nblk(4LL * cnt, 128), 128, s, A, ord, st, cnt);
+                if (!c->crowded && quad_level(cnt)) OFG_LAUNCH((k_lusgs_quad<R, false>), nblk(4LL * cnt, 128), 128, s, A, ord, st, cnt);
                 else OFG_LAUNCH(k_lusgs_upper<R>, nblk(cnt, 128), 128, s, A, ord, st, cnt);
             }
         }
