@@ -311,8 +311,7 @@ void build_lists(const ofg_ctx *c, NbLists &L) {
     }
 }
 
-// The chained sweeps' schedules (ofg_chain.cuh): edge slots [level][j-th edge][cell of the level], each edge with
-// its neighbour's place in the ring, or ~neighbour where the ring no longer (or not for the whole level) holds it.
+// The chained sweeps' schedules (plan_sweep) and their memory on the device.
 // Without the memory for them, or where a level is wider than the cluster's
 // signals can carry, the sweeps stay one launch per level.
 int build_chain(ofg_ctx *c, const NbLists *lists = nullptr) {
@@ -327,52 +326,10 @@ int build_chain(ofg_ctx *c, const NbLists *lists = nullptr) {
         lists = &own;
     }
     // the two sweeps' plans side by side
-    struct Plan {
-        std::vector<int> lev, ref, edge;
-        long long slots = 0;
-        int far = 0;
-        bool fits = true;
-    } plans[2];
+    SweepPlan plans[2];
     auto build = [&](int dir) {
-        Plan &P = plans[dir];
-        const std::vector<int> &order = dir == 0 ? c->lowOrder : c->upOrder, &off = dir == 0 ? c->lowOff : c->upOff;
-        const std::vector<int> &nbOff = dir == 0 ? lists->loOff : lists->upOff;
-        const std::vector<int> &nbl = dir == 0 ? lists->lol : lists->upl;
-        const int nlev = int(off.size()) - 1;
-        std::vector<int> pos(c->nCells), at(c->nCells);
-        P.lev.assign(4 * (size_t)nlev, 0);
-        for (int l = 0; l < nlev; ++l) {
-            int deg = 0;
-            for (int k = off[l]; k < off[l + 1]; ++k) {
-                const int i = order[k];
-                pos[i] = k; at[i] = l;
-                deg = std::max(deg, nbOff[i + 1] - nbOff[i]);
-            }
-            int *m = &P.lev[4 * (size_t)l];
-            m[0] = off[l]; m[1] = off[l + 1] - off[l]; m[2] = int(P.slots); m[3] = deg;
-            P.slots += (long long)deg * m[1];
-            P.fits = P.fits && P.slots <= INT32_MAX / 4 && m[1] <= kChainLevel;
-            if (!P.fits) return;
-        }
-        P.ref.assign(P.slots, kChainNone);
-        P.edge.assign(4 * P.slots, -1);
-        for (int l = 0; l < nlev; ++l) {
-            const int *m = &P.lev[4 * (size_t)l];
-            for (int t = 0; t < m[1]; ++t) {
-                const int i = order[m[0] + t];
-                size_t s = (size_t)m[2] + t;
-                for (int q = nbOff[i]; q < nbOff[i + 1]; ++q, s += m[1]) {   // ascending face id
-                    const int nb = nbl[2 * (size_t)q + 1];
-                    const bool near = pos[nb] + kChainRing >= off[l + 1];
-                    P.ref[s] = near ? pos[nb] & (kChainRing - 1) : ~nb;
-                    // a global copy written after its signal is safe to read
-                    // from the level after its warp's next signal on
-                    if (!near) P.far = std::max(P.far, l <= at[nb] + kChainGroups ? 2 : 1);
-                    int *e = &P.edge[4 * s];
-                    e[0] = nbl[2 * (size_t)q]; e[1] = nb; e[2] = i;
-                }
-            }
-        }
+        if (dir == 0) plan_sweep(c->nCells, c->lowOrder, c->lowOff, lists->loOff, lists->lol, plans[0]);
+        else plan_sweep(c->nCells, c->upOrder, c->upOff, lists->upOff, lists->upl, plans[1]);
     };
     auto guarded = [&](int dir) {   // no memory for a plan: no chain
         try {
@@ -395,7 +352,7 @@ int build_chain(ofg_ctx *c, const NbLists *lists = nullptr) {
     auto whole = [](size_t n) { return (n + 255) / 256 * 256; };
     size_t at[2][3], n = 0;
     for (int dir = 0; dir < 2; ++dir) {
-        const Plan &P = plans[dir];
+        const SweepPlan &P = plans[dir];
         const size_t sizes[3] = {P.lev.size(), P.edge.size(), P.ref.size()};
         for (int k = 0; k < 3; ++k) { at[dir][k] = n; n += whole(sizes[k] * sizeof(int)); }
     }
@@ -407,7 +364,7 @@ int build_chain(ofg_ctx *c, const NbLists *lists = nullptr) {
         return OFG_OK;
     }
     for (int dir = 0; dir < 2; ++dir) {
-        const Plan &P = plans[dir];
+        const SweepPlan &P = plans[dir];
         const std::vector<int> *parts[3] = {&P.lev, &P.edge, &P.ref};
         for (int k = 0; k < 3; ++k)
             CK(cudaMemcpyAsync(c->d_chain + at[dir][k], parts[k]->data(), parts[k]->size() * sizeof(int),

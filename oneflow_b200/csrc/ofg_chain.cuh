@@ -144,6 +144,11 @@ __device__ __forceinline__ void chain_cluster_sync() {
 __device__ __forceinline__ void chain_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// a cluster: the same without an order of its own (the data come with the
+// bytes; global copies are ordered by a fence ahead of it where they are read)
+__device__ __forceinline__ void chain_arrive_relaxed(uint32_t bar) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void chain_expect(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");
@@ -190,12 +195,19 @@ __device__ __forceinline__ bool chain_wait(uint32_t bar, uint32_t parity) {
 // before the wait), solve(t, m) forms the cell's increment, send(t, m, bar, n)
 // puts it in the ring of every block, store() writes its global copy.
 //
-// One block: every warp of a level arrives on the level's mbarrier.  A
-// cluster: the increments travel by st.async, which counts their bytes on the
-// receiving block's mbarrier, and every block sends one more 16-byte word to
-// every block for every level once it has seen the level before: so no block
-// can run two levels ahead of what another has received, and an mbarrier
-// never meets bytes of a later phase than its next.
+// Every warp of a level's group arrives once on its block's mbarrier of that
+// level, whether it has cells of the level or not.  One block: after its cells. A
+// cluster: as soon as it has seen the level before, since the increments travel
+// by st.async, which counts their bytes on the receiving block's mbarrier; and
+// every block sends one more 16-byte word to every block for every level. So
+// - no phase of an mbarrier completes before every warp of the block has seen the
+//   level before it, and with it the mbarrier's own last phase: a warp that
+//   lags meets the parity it waits for, and the next phase's bytes and arrivals
+//   never meet the one before;
+// - no block runs two levels ahead of what another has seen: its word of a
+//   level follows all its warps' arrivals in the level before.
+// (With the first warp's arrival alone, a warp without cells in two levels could
+// miss both and wait for a phase that waits for it.)
 template <bool CL, typename Body>
 __device__ __forceinline__ void chain_run(const ChainPlan &P, uint64_t *bars, double2 *word, Body &body) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -205,8 +217,7 @@ __device__ __forceinline__ void chain_run(const ChainPlan &P, uint64_t *bars, do
     const uint32_t bar0 = chain_smem(bars);
     if (threadIdx.x == 0) {
         for (int k = 0; k < kChainGroups; ++k)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar0 + 8 * k), "r"(CL ? 1 : kChainWarps)
-                         : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar0 + 8 * k), "r"(kChainArrivals) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -216,23 +227,28 @@ __device__ __forceinline__ void chain_run(const ChainPlan &P, uint64_t *bars, do
         const uint32_t bar = bar0 + 8 * (l % kChainGroups);
         int t = cw * 32 + lane;
         body.load(t, m);
-        bool ok = l == 0 || chain_wait<CL>(bar0 + 8 * ((l - 1) % kChainGroups), ((l - 1) / kChainGroups) & 1);
-        if (CL && ok && w == 0 && l >= kChainGroups)   // the phase before this level's, to arm the next
-            ok = chain_wait<CL>(bar, (l / kChainGroups - 1) & 1);
+        // a cluster: the mbarrier's own last phase first, so that every warp has acquired every level
+        bool ok = !CL || l < kChainGroups || chain_wait<CL>(bar, (l / kChainGroups - 1) & 1);
+        if (ok) ok = l == 0 || chain_wait<CL>(bar0 + 8 * ((l - 1) % kChainGroups), ((l - 1) / kChainGroups) & 1);
         if (!__all_sync(0xffffffffu, ok)) {            // the whole warp leaves together
             *reinterpret_cast<volatile unsigned *>(P.status) = 1u;   // pinned host memory
             break;
         }
         if (CL) {
-            if (P.far) asm volatile("fence.acq_rel.cluster;" ::: "memory");   // this warp's earlier global copies
+            if (P.far) {   // this warp's earlier global copies
+                __syncwarp();
+                asm volatile("fence.acq_rel.cluster;" ::: "memory");
+            }
             if (w == 0) {
                 if (lane == 0) chain_expect(bar, uint32_t(m.y) * Body::kBytes + 16u * n);
                 if (lane < n) chain_send(chain_peer(chain_smem(word + rank), lane), 0.0, 0.0, chain_peer(bar, lane));
+            } else if (lane == 0) {
+                chain_arrive_relaxed(bar);
             }
         }
         // a cell's global copy goes out after its signal, off the path between
-        // levels; first where a level that starts before this warp's next
-        // signal may read it
+        // levels; first where a level may read it that starts before this
+        // warp's next arrival is known to every block
         auto put = [&](int at) {
             if (P.far == 2) {
                 body.store();

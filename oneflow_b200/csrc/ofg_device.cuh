@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ofg_chain_plan.h"
+
 namespace ofg {
 
 constexpr double SMALLD = 1.0e-40;   // codes/basic/include/HXTypeBasic.h:34
@@ -44,11 +46,7 @@ template <> struct MinBlocks<float> {
 
 constexpr int kRedBlocks = 148;   // blocks of the grid reductions (one per SM)
 
-// chained sweeps (ofg_chain.cuh): warps of a level and groups of them in a block; ring positions
-constexpr int kChainWarps = 6, kChainGroups = 2, kChainThreads = 32 * kChainWarps * kChainGroups;
-constexpr int kChainRing = 4096, kChainMaxBlocks = 16;
-constexpr int kChainLevel = 16384;       // cells of a level: 64 bytes each stay below an mbarrier's 2^20 - 1
-constexpr int kChainNone = INT32_MIN;   // an empty edge slot
+// chained sweeps (ofg_chain.cuh)
 constexpr int kEdgeCoefs = 15;          // values of an edge that do not depend on the increments
 constexpr int kChainCell = NEQ + 2;     // values of a cell: right-hand side, diagonal, its reciprocal
 
