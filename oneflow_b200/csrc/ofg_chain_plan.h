@@ -31,9 +31,13 @@ struct SweepPlan {
 // order[nCells]: the cells level after level, off[levels + 1] the levels; nbOff /
 // nbl: each cell's edges in ascending face id, {face | side << 31, neighbour}.
 //
-// The ring holds position p of the level order in slot p mod kChainRing: an edge
-// of level l takes its neighbour from the ring while later positions up to the
-// end of level l have other slots.
+// The ring holds position p of the level order in slot p mod kChainRing.  Levels
+// are ordered one after the other, the cells of a level are not.  So an edge of
+// level l takes its neighbour from the ring where every other write to the slot
+// is ordered against this read:
+// - near: later positions up to the end of level l have other slots;
+// - alone: so have the earlier positions of the neighbour's own level (in a level
+//   wider than the ring their write may arrive last).
 inline void plan_sweep(int nCells, const std::vector<int> &order, const std::vector<int> &off, const std::vector<int> &nbOff,
                        const std::vector<int> &nbl, SweepPlan &P) {
     const int nlev = int(off.size()) - 1;
@@ -61,14 +65,14 @@ inline void plan_sweep(int nCells, const std::vector<int> &order, const std::vec
             size_t s = (size_t)m[2] + t;
             for (int q = nbOff[i]; q < nbOff[i + 1]; ++q, s += m[1]) {   // ascending face id
                 const int nb = nbl[2 * (size_t)q + 1];
-                const bool near = pos[nb] + kChainRing >= off[l + 1];
-                P.ref[s] = near ? pos[nb] & (kChainRing - 1) : ~nb;
+                const bool near = pos[nb] + kChainRing >= off[l + 1], alone = pos[nb] - kChainRing < off[at[nb]];
+                P.ref[s] = near && alone ? pos[nb] & (kChainRing - 1) : ~nb;
                 // A global copy written after its signal, in level a, is
                 // released by its warp's next arrival, in level a +
                 // kChainGroups; the other blocks learn of that arrival by
                 // the word its block sends in the level after, so their
                 // cells may read the copy from the level after that on.
-                if (!near) P.far = std::max(P.far, l <= at[nb] + kChainGroups + 1 ? 2 : 1);
+                if (P.ref[s] < 0) P.far = std::max(P.far, l <= at[nb] + kChainGroups + 1 ? 2 : 1);
                 int *e = &P.edge[4 * s];
                 e[0] = nbl[2 * (size_t)q]; e[1] = nb; e[2] = i;
             }

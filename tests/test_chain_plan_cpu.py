@@ -1,6 +1,10 @@
 """The chained sweeps' schedules (oneflow_b200/csrc/ofg_chain_plan.h), compiled
 for the host: every edge names its neighbour, in the ring or in global memory, and
-a neighbour read from global memory is written early enough.  And the cluster's
+a neighbour read from global memory is written early enough.  Where it names a ring
+slot, no write to that slot is unordered against the read: levels are ordered one
+after the other, the cells of a level are not, so what a slot holds is decided only
+if the neighbour's is the one position of its level with that slot, and no position
+of a later level up to the reader's own has it.  And the cluster's
 phases, replayed with warps that lag: every wait ends."""
 import ctypes as C
 import os
@@ -92,7 +96,9 @@ def mesh_of(name):
     return m
 
 
-NAMES = ["plate2d", "bump-33-21", "bump-60-40-shuffled", "bump-70-50-shuffled"]
+# the widest levels: 30 and 33 cells, 1,300, 1,900; 4,200 and 7,600, wider than the ring
+NAMES = ["plate2d", "bump-33-21", "bump-60-40-shuffled", "bump-70-50-shuffled", "bump-110-70-shuffled",
+         "bump-140-100-shuffled"]
 
 
 @pytest.mark.parametrize("name", NAMES)
@@ -116,6 +122,30 @@ def test_every_edge_finds_its_neighbour(lib, name, lower):
     # levels on, and known to the other blocks a level after that
     late = lev[cell[~near]] > lev[nb[~near]] + lib.groups() + 1
     assert far == (0 if near.all() else 1 if late.all() else 2)
+
+
+@pytest.mark.parametrize("name", NAMES)
+@pytest.mark.parametrize("lower", [True, False])
+def test_no_slot_of_the_ring_is_read_with_an_unordered_write(lib, name, lower):
+    sw = sweep(mesh_of(name), lower)
+    lev, order = sw[:2]
+    m, ref, edge, _ = plan(lib, sw)
+    n, ring = len(order), lib.ring()
+    pos = np.empty(n, np.int64)
+    pos[order] = np.arange(n)
+    near = np.flatnonzero((edge[:, 1] >= 0) & (ref >= 0))
+    for c, q in zip(edge[near, 2], edge[near, 1]):
+        p = int(pos[q])
+        others = np.arange(p % ring, n, ring)
+        others = others[others != p]
+        at = lev[order[others]]
+        # the other writers of the slot: none in the neighbour's level, none after it up to the reader's level
+        assert not ((at >= lev[q]) & (at <= lev[c])).any(), (c, q)
+
+
+def test_levels_wider_than_the_ring_are_among_them(lib):
+    widest = [np.diff(sweep(mesh_of(n), True)[2]).max() for n in NAMES]
+    assert sum(w > lib.ring() for w in widest) == 2 and min(widest) < 100
 
 
 def test_a_read_three_levels_on_is_among_them(lib):

@@ -1,13 +1,14 @@
 """The chained LU-SGS sweeps in a cluster of blocks on level structures that try
 their orders: levels of one cell between levels that occupy every warp, and
 neighbours that the ring no longer holds, read a few levels after they were
-written.  Against one launch per level: the same bits."""
+written, and levels wider than the ring, whose cells share its slots.  Against one launch per level: the same bits."""
 import numpy as np
 import pytest
 
 from oneflow_b200 import meshgen, params as P
 from oneflow_b200.meshio import Mesh
-from oneflow_b200.solver import Solver
+from oneflow_b200.solver import TURB_SOLVER, Solver
+from oneflow_b200.walldist import plate_wall_distance
 
 pytestmark = pytest.mark.gpu
 
@@ -52,7 +53,7 @@ def both(m, prm, steps=4):
         s.set_tuning(sweep_persistent=chained)
         s.init_flowfield()
         s.step(steps)
-        got.append([s.state(), s.res_history()])
+        got.append([s.state(), s.res_history()] + ([s.state(TURB_SOLVER)] if prm.vismodel >= 3 else []))
         s.close()
     assert np.isfinite(got[0][0]).all()
     for a, b in zip(*got):
@@ -67,3 +68,17 @@ def test_levels_of_one_cell_between_wide_ones(width, rows, precision):
 @pytest.mark.parametrize("precision", [0, 1])
 def test_neighbours_beyond_the_ring_a_few_levels_on(precision):
     both(shuffled(meshgen.bump_channel(60, 40), 20), P.euler_bump(precision=precision, ilim=2, vencat_coef=0.05))
+
+
+@pytest.mark.parametrize("name", ["bump_4k", "bump_7k", "bump_mixed", "ladder", "plate3d", "plate3d_fp64"])
+def test_levels_wider_than_the_ring(name):
+    """widest levels of 4,200 to 12,400 cells, narrower ones after them"""
+    if name == "ladder":   # its upper sweep begins with one level of half the quadrilaterals
+        return both(ladder(3100, 8), P.euler_bump())
+    if name.startswith("bump"):
+        ni, nj, precision = {"bump_4k": (110, 70, 0), "bump_7k": (140, 100, 0), "bump_mixed": (140, 100, 1)}[name]
+        return both(shuffled(meshgen.bump_channel(ni, nj), 21),
+                    P.euler_bump(precision=precision, ilim=2, vencat_coef=0.05))
+    m = meshgen.flat_plate_tets(26, 16, 10)
+    m.wall_dist = plate_wall_distance(m)
+    both(shuffled(m, 1), P.rans_plate(precision=0 if name == "plate3d_fp64" else 1, sweep_order=0))
