@@ -274,7 +274,15 @@ __device__ __forceinline__ void chain_run(const ChainPlan &P, uint64_t *bars, do
             if (P.far != 2 && mine) body.store();   // the last cell's
         }
     }
-    if (CL) chain_cluster_sync();   // no block leaves while another may still write to its ring
+    if (CL) {
+        // no block leaves while increments of the last level, which nobody
+        // waited for, may still be on their way to its ring: a block sees
+        // its own in, then all blocks leave together
+        if (warp == 0 && !chain_wait<CL>(bar0 + 8 * ((P.nlev - 1) % kChainGroups), ((P.nlev - 1) / kChainGroups) & 1))
+            *reinterpret_cast<volatile unsigned *>(P.status) = 1u;
+        __syncwarp();
+        chain_cluster_sync();
+    }
 }
 
 // One sweep of the NS increments.  LOWER: dq = (res - rhs0) / rad; else the
