@@ -271,6 +271,22 @@ bool chain_pays(const ofg_ctx *c) {
     return nlev >= 16 && c->nCells / nlev <= 1024;
 }
 
+// Memory that only buys speed -- the chained sweeps' schedules, the second set of
+// gradient records -- is taken after everything a solve cannot do without, and
+// only while half of the device's memory stays free, for what else the caller
+// puts there.
+bool spare_memory(size_t bytes) {
+    size_t free = 0, total = 0;
+    return cudaMemGetInfo(&free, &total) == cudaSuccess && free > bytes && free - bytes >= total / 2;
+}
+
+// Whether an SA iteration overlapped with the next one's gradients (kSteps) is
+// worth a second set of their records: where a pass by itself keeps memory busy
+// it is not.  Measured, us an iteration without / with: mixed 600,000 468.0 / 458.1,
+// 1,200,000 860 / 859, 2,400,000 1,622 / 1,626, 3,600,000 2,349 / 2,360; FP64
+// 312,500 604.6 / 568.9, 1,200,000 1,943 / 1,929, 2,400,000 3,770 / 3,781.
+bool overlap_pays(int cells) { return cells <= 1500000; }
+
 void free_chain(ofg_ctx *c) {
     cudaFree(c->d_chain);   // holds both plans
     c->d_chain = nullptr;
@@ -322,7 +338,11 @@ int build_chain(ofg_ctx *c, const NbLists *lists = nullptr) {
     }
     NbLists own;
     if (!lists) {
-        build_lists(c, own);
+        try {
+            build_lists(c, own);
+        } catch (const std::exception &) {   // no memory for them: no chain
+            return OFG_OK;
+        }
         lists = &own;
     }
     // the two sweeps' plans side by side
@@ -358,6 +378,7 @@ int build_chain(ofg_ctx *c, const NbLists *lists = nullptr) {
     }
     const size_t coef = n + whole((size_t)kChainCell * c->nCells * sizeof(double));
     const size_t bytes = coef + whole((size_t)std::max(plans[0].slots, plans[1].slots) * kEdgeCoefs * real);
+    if (!spare_memory(bytes)) return OFG_OK;
     if (cudaMalloc((void **)&c->d_chain, bytes) != cudaSuccess) {
         cudaGetLastError();
         c->d_chain = nullptr;
@@ -618,9 +639,12 @@ int ofg_upload_mesh(ofg_ctx *c, int nNodes, const double *xN, const double *yN, 
     // ---- device copies ----
     int rc;
     const bool mixed = c->p.precision == OFG_PREC_MIXED;
+    free_chain(c);
+    if (c->d_gl[1]) { cudaFree(c->d_gl[1]); c->d_gl[1] = nullptr; }
+    c->gl = 0;
+    NbLists L;
+    build_lists(c, L);
     {
-        NbLists L;
-        build_lists(c, L);
         std::vector<int> lcb(c->lc.begin(), c->lc.begin() + nBFaces);
         if ((rc = upload(c, &c->d_lcb, lcb.data(), nBFaces))) return rc;
         if ((rc = upload(c, &c->d_nb_off, L.nbOff.data(), L.nbOff.size()))) return rc;
@@ -629,9 +653,6 @@ int ofg_upload_mesh(ofg_ctx *c, int nNodes, const double *xN, const double *yN, 
         if ((rc = upload(c, &c->d_lol, L.lol.data(), L.lol.size()))) return rc;
         if ((rc = upload(c, &c->d_up_off, L.upOff.data(), L.upOff.size()))) return rc;
         if ((rc = upload(c, &c->d_upl, L.upl.data(), L.upl.size()))) return rc;
-        free_chain(c);
-        if (!c->tuneSet) c->tune.sweep_persistent = chain_pays(c) ? 1 : 0;
-        if (c->tune.sweep_persistent && !multi_stage(c) && (rc = build_chain(c, &L))) return rc;
     }
     // metrics on the GPU (UnsGrid::CalcMetrics); for an SA solve without a
     // caller-supplied wall distance, CALC_WALL_DIST on the GPU as well
@@ -736,12 +757,6 @@ int ofg_upload_mesh(ofg_ctx *c, int nNodes, const double *xN, const double *yN, 
     if ((rc = upload<double>(c, &c->d_hist, nullptr, (size_t)c->histCap * NEQ))) return rc;
     if ((rc = upload<int>(c, &c->d_fix, nullptr, 1 + c->fixcap))) return rc;
     if ((rc = upload_bytes(c, &c->d_gl[0], nullptr, N * GLR * rs))) return rc;
-    if (c->d_gl[1]) { cudaFree(c->d_gl[1]); c->d_gl[1] = nullptr; }
-    c->gl = 0;
-    if (has_turb(c) && cudaMalloc(&c->d_gl[1], N * GLR * rs) != cudaSuccess) {   // then the iterations do not overlap
-        cudaGetLastError();
-        c->d_gl[1] = nullptr;
-    }
     bool venkatGlobal = c->p.ilim == 2 && !c->p.venkat_kh3;
     if ((rc = upload_bytes(c, &c->d_mm, nullptr, venkatGlobal ? N * MMR * rs : 0))) return rc;
     CK(cudaMemset(c->d_bcq, 0, (size_t)std::max(nBFaces, 1) * NEQ * sizeof(double)));
@@ -759,6 +774,14 @@ int ofg_upload_mesh(ofg_ctx *c, int nNodes, const double *xN, const double *yN, 
         if ((rc = upload<double>(c, &c->d_thist, nullptr, c->histCap))) return rc;
         if ((rc = upload_bytes(c, &c->d_gnut, nullptr, N * 4 * rs))) return rc;
         CK(cudaMemset(c->d_dnut, 0, nT * sizeof(double)));
+    }
+    // what the solve can do without comes last
+    if (!c->tuneSet) c->tune.sweep_persistent = chain_pays(c) ? 1 : 0;
+    if (c->tune.sweep_persistent && !multi_stage(c) && (rc = build_chain(c, &L))) return rc;
+    if (has_turb(c) && overlap_pays(nCells) && spare_memory(N * GLR * rs) &&
+        cudaMalloc(&c->d_gl[1], N * GLR * rs) != cudaSuccess) {   // then the iterations do not overlap
+        cudaGetLastError();
+        c->d_gl[1] = nullptr;
     }
     c->haveMesh = true;
     c->haveState = false;
@@ -1052,9 +1075,9 @@ int ofg_calc_boundary(ofg_ctx *c, int tid) {
 // iteration has none, and is launched as it stands while the graphs run (a third
 // and fourth graph cost a new solver 0.6 ms).  Measured, us an iteration in one chain /
 // overlapped: 600,000 tetrahedra (mixed) 468.0 / 458.1, 769,000 cells (mixed)
-// 630.4 / 618.1, 312,500 cells (FP64) 604.6 / 568.9; at 6 million (mixed), where
-// each pass by itself keeps memory busy, 3946 / 3944.  Begun later, beside the
-// sweeps alone, the gradients gained less (FP64: 583.5).
+// 630.4 / 618.1, 312,500 cells (FP64) 604.6 / 568.9; overlap_pays has the larger
+// meshes, where it does not pay.  Begun later, beside the sweeps alone, the
+// gradients gained less (FP64: 583.5).
 enum Fork { F_MAIN, F_FORK, F_SIDE, F_JOIN };   // a task of the chain; the branch's start, a task of it, its end
 enum Stage { S_NS, S_SA, S_NEXT };              // the task's state: the iteration's, the updated one (SA; the next gradients)
 enum Need { N_ALWAYS, N_SA, N_FULL, N_MORE };   // only with an SA solver; only in a whole iteration's graph; only
