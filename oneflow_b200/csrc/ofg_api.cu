@@ -1796,8 +1796,9 @@ int ofg_set_tuning(ofg_ctx *c, const ofg_tuning *t) {
     n.ms_default = c->tune.ms_default; n.ms_tuned = c->tune.ms_tuned;
     c->tune = n;
     c->tuneSet = true;
-    if (n.sweep_persistent && c->haveMesh && (rc = build_chain(c))) return rc;
     destroy_graphs(c);   // recaptured with the new kernels at the next ofg_step
+    if (!n.sweep_persistent) free_chain(c);
+    else if (c->haveMesh && (rc = build_chain(c))) return rc;
     return OFG_OK;
 }
 
@@ -1862,43 +1863,67 @@ int ofg_autotune(ofg_ctx *c, int reps, ofg_tuning *out) {
     // groups in turn, each over its own candidates, the others at their current choice
     struct Cand { int *a; int *b; std::vector<std::pair<int, int>> values; std::vector<int> tasks; };
     ofg_tuning &T = c->tune;
-    std::vector<Cand> groups;
-    if (mixed) {
-        groups.push_back({&T.face_min_blocks, &T.face_block,
-                          {{2, 128}, {3, 128}, {4, 128}, {5, 128}, {2, 64}, {3, 64}, {4, 64}, {5, 64}}, {T_P_FLUX}});
-        groups.push_back({&T.grad_min_blocks, &T.grad_block,
-                          {{4, 128}, {6, 128}, {8, 128}, {4, 64}, {6, 64}, {8, 64}}, {T_P_GRADLIM}});
-        groups.push_back({&T.sweep_min_blocks, &T.sweep_block,
-                          {{6, 128}, {8, 128}, {10, 128}, {6, 64}, {8, 64}, {10, 64}}, {T_LOWER, T_UPPER}});
-    }
-    // the sweep schedule: level launches or the chained form (not tried when
-    // the levels average more than 4,096 cells: one cluster cannot keep up
-    // with a full-width level launch there)
-    const int nlev = std::max<int>(1, int(c->lowOff.size()) - 1);
-    if (c->nCells / nlev <= 4096) {
-        if ((rc = build_chain(c))) return rc;
-        groups.push_back({&T.sweep_persistent, nullptr, {{0, 0}, {1, 0}}, {T_LOWER, T_UPPER}});
-    }
-    for (Cand &g : groups) {
+    // first: the time of the shape the context came with; best: the chosen one's
+    auto tune_group = [&](const Cand &g, double &first, double &best) -> int {
         const int a0 = *g.a, b0 = g.b ? *g.b : 0;
-        double best = 1e30, first = 0.0;
         int ba = a0, bb = b0;
-        for (size_t k = 0; k < g.values.size(); ++k) {
-            *g.a = g.values[k].first;
-            if (g.b) *g.b = g.values[k].second;
+        best = 1e30;
+        for (const auto &v : g.values) {
+            *g.a = v.first;
+            if (g.b) *g.b = v.second;
             double ms = 0.0;
-            std::vector<int> tl(g.tasks);
-            int q;
-            if (tl.size() == 1) q = time_group({tl[0]}, ms);
-            else q = time_group({tl[0], tl[1]}, ms);
-            if (q) { cudaEventDestroy(e0); cudaEventDestroy(e1); c->tune = start; return q; }
-            if (*g.a == a0 && (!g.b || *g.b == b0)) first = ms;   // the shape the context came with
+            const int q = g.tasks.size() == 1 ? time_group({g.tasks[0]}, ms) : time_group({g.tasks[0], g.tasks[1]}, ms);
+            if (q) return q;
+            if (*g.a == a0 && (!g.b || *g.b == b0)) first = ms;
             if (ms < best) { best = ms; ba = *g.a; bb = g.b ? *g.b : 0; }
         }
         *g.a = ba;
         if (g.b) *g.b = bb;
-        msDefault += first;
-        msTuned += best;
+        return OFG_OK;
+    };
+    auto quit = [&](int q) {
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        c->tune = start;
+        return q;
+    };
+    if (mixed) {
+        const Cand gathers[] = {
+            {&T.face_min_blocks, &T.face_block,
+             {{2, 128}, {3, 128}, {4, 128}, {5, 128}, {2, 64}, {3, 64}, {4, 64}, {5, 64}}, {T_P_FLUX}},
+            {&T.grad_min_blocks, &T.grad_block,
+             {{4, 128}, {6, 128}, {8, 128}, {4, 64}, {6, 64}, {8, 64}}, {T_P_GRADLIM}}};
+        for (const Cand &g : gathers) {
+            double first = 0.0, best = 0.0;
+            if ((rc = tune_group(g, first, best))) return quit(rc);
+            msDefault += first;
+            msTuned += best;
+        }
+    }
+    // the sweeps: the shape of their level launches first (the chained form has
+    // none), then the schedule -- level launches of that shape or the chained form,
+    // which is not tried when the levels average more than 4,096 cells (one
+    // cluster cannot keep up with a full-width level launch there), unless the
+    // context came with it
+    const int nlev = std::max<int>(1, int(c->lowOff.size()) - 1);
+    const bool chain = c->nCells / nlev <= 4096 || start.sweep_persistent;
+    if (chain && (rc = build_chain(c))) return quit(rc);
+    const bool built = c->chain[0].lev && c->chain[1].lev;
+    if (mixed || chain) {
+        T.sweep_persistent = 0;
+        double first = 0.0, level = 0.0, chained = 1e30;
+        const Cand shapes{&T.sweep_min_blocks, &T.sweep_block,
+                          {{6, 128}, {8, 128}, {10, 128}, {6, 64}, {8, 64}, {10, 64}}, {T_LOWER, T_UPPER}};
+        if (mixed) rc = tune_group(shapes, first, level);
+        else if (!(rc = time_group({T_LOWER, T_UPPER}, level))) first = level;
+        if (!rc && chain && built) {
+            T.sweep_persistent = 1;
+            rc = time_group({T_LOWER, T_UPPER}, chained);
+        }
+        if (rc) return quit(rc);
+        T.sweep_persistent = chained < level ? 1 : 0;
+        msDefault += start.sweep_persistent && built ? chained : first;
+        msTuned += std::min(level, chained);
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -1906,12 +1931,14 @@ int ofg_autotune(ofg_ctx *c, int reps, ofg_tuning *out) {
     T.ms_tuned = msTuned;
     c->tuneSet = true;
     destroy_graphs(c);
+    if ((rc = sync(c))) return rc;
+    if (!T.sweep_persistent) free_chain(c);
     {
         std::lock_guard<std::mutex> g(g_tuneMutex);
         g_tuneCache[key] = T;
     }
     if (out) *out = T;
-    return sync(c);
+    return OFG_OK;
 }
 
 int ofg_colour_order(int nCells, int nFaces, int nBFaces, const int *lCells, const int *rCells, int *perm) {
