@@ -70,6 +70,14 @@ __device__ __forceinline__ void ld8(const float *p, float *o) {
         : "l"(p));
 }
 __device__ __forceinline__ void ld8(const double *p, double *o) { ld4(p, o); ld4(p + 4, o + 4); }
+// A state record for the gradients: its last word, the eddy viscosity, may be
+// written by the SA stage that runs beside them (put_vist).  They do not use it, but
+// a read-only load may only touch what nothing writes during the kernel: the
+// half that holds it comes by a plain load of the same width.
+__device__ __forceinline__ void ld_state(const double *p, double *o) {
+    ld4(p, o);
+    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(o[4]), "=d"(o[5]), "=d"(o[6]), "=d"(o[7]) : "l"(p + 4));
+}
 // plain (coherent) vector loads, for a record the same launch writes afterwards
 __device__ __forceinline__ void ldp8(const float *p, float *o) {
     asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -328,7 +336,7 @@ __global__ void __launch_bounds__(128, MINB) k_gradlim(KArgs<R> A, int nvar, int
     constexpr bool mixed = sizeof(R) == 4;
     if (active) {
         R qc[REC], cgc[CGR];
-        if constexpr (!mixed) ld8(A.qs + (size_t)c * REC, qc);
+        if constexpr (!mixed) ld_state(A.q + (size_t)c * REC, qc);
         ld4(A.cgeo + (size_t)c * CGR, cgc);
         R gx[6], gy[6], gz[6];
 #pragma unroll
@@ -348,7 +356,7 @@ __global__ void __launch_bounds__(128, MINB) k_gradlim(KArgs<R> A, int nvar, int
                 R dx, dy, dz;
                 if constexpr (mixed) {
                     double t[REC];
-                    ld8(A.q + (size_t)nb * REC, t);
+                    ld_state(A.q + (size_t)nb * REC, t);
 #pragma unroll
                     for (int v = 0; v < 6; ++v)   // the cell's own values re-read (L1 hits), not held
                         dn[v] = R(t[v < 5 ? v : ITT] - __ldg(A.q + (size_t)c * REC + (v < 5 ? v : ITT)));
@@ -358,7 +366,7 @@ __global__ void __launch_bounds__(128, MINB) k_gradlim(KArgs<R> A, int nvar, int
                     const float sg = nb_right(e2) ? -1.0f : 1.0f;
                     dx = sg * (fo[0] - fo[3]); dy = sg * (fo[1] - fo[4]); dz = sg * (fo[2] - fo[5]);
                 } else {
-                    ld8(A.qs + (size_t)nb * REC, qn);
+                    ld_state(A.q + (size_t)nb * REC, qn);
 #pragma unroll
                     for (int v = 0; v < 6; ++v) dn[v] = qn[v < 5 ? v : ITT] - qc[v < 5 ? v : ITT];
                     ld4(A.cgeo + (size_t)nb * CGR, cgn);
@@ -409,7 +417,7 @@ __global__ void __launch_bounds__(128, MINB) k_gradlim(KArgs<R> A, int nvar, int
                 R cl, cr;
                 if constexpr (mixed) {
                     double t[REC];
-                    ld8(A.q + (size_t)nb * REC, t);
+                    ld_state(A.q + (size_t)nb * REC, t);
 #pragma unroll
                     for (int v = 0; v < 6; ++v)   // the cell's own values re-read (L1 hits), not held
                         dn[v] = R(t[v < 5 ? v : ITT] - __ldg(A.q + (size_t)c * REC + (v < 5 ? v : ITT)));
@@ -422,7 +430,7 @@ __global__ void __launch_bounds__(128, MINB) k_gradlim(KArgs<R> A, int nvar, int
                         cl = dd.y * delta; cr = dd.x * delta;
                     }
                 } else {
-                    ld8(A.qs + (size_t)nb * REC, qn);
+                    ld_state(A.q + (size_t)nb * REC, qn);
                     ld4(A.cgeo + (size_t)nb * CGR, cgn);
                     ld8(A.fgeo + (size_t)f * FGR, fg);
                     const R *cl_ = right ? cgn : cgc, *cr_ = right ? cgc : cgn;
