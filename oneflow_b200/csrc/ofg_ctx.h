@@ -117,7 +117,7 @@ enum Task {
     T_FORCES, T_GRAD_ONLY, T_CALC_LHS,
     // the fused iteration's: on meshes where it pays the lower sweep's first
     // level runs with the diagonal; the update starts the next outer step
-    T_CLIP0, T_LOWER1, T_UPDATE_NEXT, T_GRADLIM0
+    T_CLIP0, T_LOWER1, T_UPDATE_NEXT, T_GRADLIM0, T_BEGIN
 };
 int launch_task_f64(ofg_ctx *c, int task, cudaStream_t s);
 int launch_task_f32(ofg_ctx *c, int task, cudaStream_t s);

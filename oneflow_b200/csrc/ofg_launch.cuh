@@ -17,6 +17,14 @@ static __global__ void k_cfl(double *scal, long long *ext, double step, Ramp ram
     start_step(scal, ext, step < 0 ? scal[S_STEP] + 1.0 : step, ramp);
 }
 
+// before n fused iterations: the counters follow the host's, and the first outer step starts (not the multi-stage
+// scheme's, whose iterations start their own)
+static __global__ void k_begin(double *scal, long long *ext, double done, bool start, Ramp ramp) {
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    scal[S_STEP] = scal[S_HISTN] = scal[S_THISTN] = done;
+    if (start) start_step(scal, ext, done + 1.0, ramp);
+}
+
 static __global__ void k_clear_extremes(long long *ext) {
     if (threadIdx.x == 0) clear_extremes(ext);
 }
@@ -226,6 +234,10 @@ int launch_task(ofg_ctx *c, int task, cudaStream_t s) {
     }
     case T_ADVANCE: {
         OFG_LAUNCH(k_cfl, 1, 32, s, c->d_scal, c->d_ext, -1.0, ramp);
+        break;
+    }
+    case T_BEGIN: {
+        OFG_LAUNCH(k_begin, 1, 32, s, c->d_scal, c->d_ext, double(c->outerSteps), c->p.time_integral != 1, ramp);
         break;
     }
     case T_TIMESTEP: {   // CALC_TIME_STEP alone (after T_CFL, which resets the minimum)
