@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -280,12 +281,24 @@ bool spare_memory(size_t bytes) {
     return cudaMemGetInfo(&free, &total) == cudaSuccess && free > bytes && free - bytes >= total / 2;
 }
 
-// Whether an SA iteration overlapped with the next one's gradients (kSteps) is
-// worth a second set of their records: where a pass by itself keeps memory busy
-// it is not.  Measured, us an iteration without / with: mixed 600,000 468.0 / 458.1,
-// 1,200,000 860 / 859, 2,400,000 1,622 / 1,626, 3,600,000 2,349 / 2,360; FP64
-// 312,500 604.6 / 568.9, 1,200,000 1,943 / 1,929, 2,400,000 3,770 / 3,781.
-bool overlap_pays(int cells) { return cells <= 1500000; }
+// The iterations of a call from which on it pays to run them overlapped with the
+// next one's gradients (kSteps), INT_MAX where it never does.  The last iteration,
+// launched as it stands, costs a call 40-55 us; and where a pass by itself keeps
+// memory busy (large meshes, FP32 least squares already at 36,000 cells) nothing is
+// gained.  Measured, us a call without / with.  FP64, 5 and 20 iterations: tetrahedra
+// 18,000 608 / 592, 2,382 / 2,158; 36,000 682 / 701, 2,677 / 2,595; 72,000 1,048 / 1,026,
+// 4,141 / 3,868; 288,000 2,830 / 2,746, 11,238 / 10,680; 600,000 5,240 / 5,182, 20,651 / 20,424;
+// airfoil of 63,220 643 / 662, 2,520 / 2,503.  Mixed, 5, 10 and 20 iterations: airfoil of
+// 44,652 364 / 369, 715 / 689, 1,410 / 1,323; wing of 179,760 1,155 / 1,152, 2,296 / 2,251,
+// 4,581 / 4,417, of 768,640 3,146 / 3,145, 6,279 / 6,240, 12,537 / 12,397; tetrahedra with
+// least squares 25,920 495 / 514, 979 / 969, 1,942 / 1,869; 36,000 491 / 523, 964 / 984,
+// 1,915 / 1,907; 72,000 592 / 662, 1,167 / 1,266, 2,315 / 2,469.  At 1.2 to 3.6 M cells
+// both paths -0.6 to +0.7 % an iteration.
+int overlap_from(const ofg_ctx *c) {
+    if (!has_turb(c) || multi_stage(c) || c->nCells > 1000000) return INT_MAX;
+    if (c->p.precision != OFG_PREC_MIXED) return c->nCells > 25000 && c->nCells <= 65000 ? 10 : 5;
+    return c->p.igrad == 2 && c->nCells > 30000 ? INT_MAX : 10;
+}
 
 void free_chain(ofg_ctx *c) {
     cudaFree(c->d_chain);   // holds both plans
@@ -778,7 +791,7 @@ int ofg_upload_mesh(ofg_ctx *c, int nNodes, const double *xN, const double *yN, 
     // what the solve can do without comes last
     if (!c->tuneSet) c->tune.sweep_persistent = chain_pays(c) ? 1 : 0;
     if (c->tune.sweep_persistent && !multi_stage(c) && (rc = build_chain(c, &L))) return rc;
-    if (has_turb(c) && overlap_pays(nCells) && spare_memory(N * GLR * rs) &&
+    if (overlap_from(c) < INT_MAX && spare_memory(N * GLR * rs) &&
         cudaMalloc(&c->d_gl[1], N * GLR * rs) != cudaSuccess) {   // then the iterations do not overlap
         cudaGetLastError();
         c->d_gl[1] = nullptr;
@@ -1073,11 +1086,10 @@ int ofg_calc_boundary(ofg_ctx *c, int tid) {
 // conditions: all wait on memory with the SMs' issue slots mostly empty.  The
 // gradients of a call's first iteration run ahead of its graph; its last
 // iteration has none, and is launched as it stands while the graphs run (a third
-// and fourth graph cost a new solver 0.6 ms).  Measured, us an iteration in one chain /
-// overlapped: 600,000 tetrahedra (mixed) 468.0 / 458.1, 769,000 cells (mixed)
-// 630.4 / 618.1, 312,500 cells (FP64) 604.6 / 568.9; overlap_pays has the larger
-// meshes, where it does not pay.  Begun later, beside the sweeps alone, the
-// gradients gained less (FP64: 583.5).
+// and fourth graph cost a new solver 0.6 ms).  overlap_from says where that pays.
+// Begun later, beside the sweeps alone, the gradients gained less (FP64, 312,500
+// cells, us an iteration in one chain / beside the SA stage / beside its sweeps:
+// 604.6 / 568.9 / 583.5).
 enum Fork { F_MAIN, F_FORK, F_SIDE, F_JOIN };   // a task of the chain; the branch's start, a task of it, its end
 enum Stage { S_NS, S_SA, S_NEXT };              // the task's state: the iteration's, the updated one (SA; the next gradients)
 enum Need { N_ALWAYS, N_SA, N_FULL, N_MORE };   // only with an SA solver; only in a whole iteration's graph; only
@@ -1097,8 +1109,6 @@ static const Step kSteps[] = {
     {F_FORK, 0, S_SA, N_SA}, {F_SIDE, T_TURB_NORM, S_SA, N_SA},
     {F_MAIN, T_TURB_LOWER, S_SA, N_SA}, {F_MAIN, T_TURB_UPPER, S_SA, N_SA}, {F_MAIN, T_TURB_UPDATE, S_SA, N_SA},
     {F_MAIN, T_TURB_BOUNDARY, S_SA, N_SA}, {F_JOIN, 0, S_SA, N_SA}};
-
-static bool overlaps(const ofg_ctx *c) { return has_turb(c) && !multi_stage(c) && c->d_gl[1]; }
 
 static int sync_history(ofg_ctx *c) {
     size_t have = c->hist.size() / NEQ;
@@ -1252,7 +1262,7 @@ static void account_step(ofg_ctx *c, GraphKind kind = G_WHOLE) {
 int ofg_step(ofg_ctx *c, int nsteps) {
     int rc = prepare_steps(c, nsteps);
     if (rc) return rc;
-    const bool overlap = overlaps(c) && nsteps > 1;
+    const bool overlap = c->d_gl[1] && nsteps >= overlap_from(c);
     if ((rc = ensure_graphs(c, overlap ? G_MORE : G_WHOLE))) return rc;
     if (overlap) {   // the first iteration's gradients
         c->gl = c->cur;

@@ -1,14 +1,14 @@
 """The sweep schedule among a context's other choices: the autotuner times the
 level kernels' shapes with level launches whatever the context came with; a
 schedule that is not in use holds no memory; a second mesh uploaded into a
-context tuned to the chained sweeps; a caller's stream around the overlapped SA
-iteration."""
+context tuned to the chained sweeps.  The overlapped SA iteration of calls of ten and
+more: against whole iterations, and around a caller's stream."""
 import numpy as np
 import pytest
 import torch
 
 from oneflow_b200 import meshgen, params as P
-from oneflow_b200.solver import TURB_SOLVER, Solver
+from oneflow_b200.solver import TURB_SOLVER, Batch, Solver
 from oneflow_b200.walldist import plate_wall_distance
 
 pytestmark = pytest.mark.gpu
@@ -85,7 +85,7 @@ def test_a_callers_stream_around_the_overlapped_iteration(order, precision):
     big = torch.empty(1 << 26, device="cuda")
     a.init_flowfield()
     b.init_flowfield()
-    for k, n in enumerate((1, 3, 2, 2)):   # the caller's streams in turn, then the context's own again
+    for k, n in enumerate((1, 10, 12, 11)):   # the caller's streams in turn, then the context's own again
         if k < 3:
             st = streams[k % 2]
             b.set_stream(st.cuda_stream)
@@ -99,3 +99,25 @@ def test_a_callers_stream_around_the_overlapped_iteration(order, precision):
         assert np.array_equal(a.state(TURB_SOLVER), b.state(TURB_SOLVER))
         assert np.array_equal(a.field("dqdx"), b.field("dqdx"))
     assert np.array_equal(a.res_history(), b.res_history())
+
+
+@pytest.mark.parametrize("order,precision,igrad", [(1, 1, 2), (1, 1, 0), (0, 1, 0), (1, 0, 0), (0, 0, 2)])
+def test_overlapped_calls_are_the_whole_iterations(order, precision, igrad):
+    """Calls long enough to be overlapped, shorter ones and odd and even numbers of
+    iterations between them, against a batch of the one solve, which runs whole ones."""
+    m, prm = plate(12, 9, 5, order, precision)
+    prm.igrad = igrad
+    a, b = Solver(m, prm), Solver(m, prm)
+    a.init_flowfield()
+    b.init_flowfield()
+    batch = Batch([b])
+    for n in (10, 1, 11, 2, 12):
+        a.step(n)
+        batch.step(n)
+        assert np.array_equal(a.state(), b.state())
+        assert np.array_equal(a.state(TURB_SOLVER), b.state(TURB_SOLVER))
+        assert np.array_equal(a.forces(), b.forces())
+        for field in ("dqdx", "dqdz", "limiter"):
+            assert np.array_equal(a.field(field), b.field(field))
+    assert np.array_equal(a.res_history(), b.res_history())
+    batch.close()
