@@ -273,12 +273,12 @@ bool chain_pays(const ofg_ctx *c) {
 }
 
 // Memory that only buys speed -- the chained sweeps' schedules, the second set of
-// gradient records -- is taken after everything a solve cannot do without, and
-// only while half of the device's memory stays free, for what else the caller
-// puts there.
-bool spare_memory(size_t bytes) {
+// gradient records -- is taken only while half of the device's memory stays free, for
+// what else the caller puts there; `later`: what this context has still to allocate.
+constexpr size_t kCellBytes = 4096;   // a cell's other arrays: measured 0.9 KB (triangles) to 1.1 KB (tetrahedra, FP64, SA)
+bool spare_memory(size_t bytes, size_t later = 0) {
     size_t free = 0, total = 0;
-    return cudaMemGetInfo(&free, &total) == cudaSuccess && free > bytes && free - bytes >= total / 2;
+    return cudaMemGetInfo(&free, &total) == cudaSuccess && free > bytes + later && free - bytes - later >= total / 2;
 }
 
 // The iterations of a call from which on it pays to run them overlapped with the
@@ -341,9 +341,10 @@ void build_lists(const ofg_ctx *c, NbLists &L) {
 }
 
 // The chained sweeps' schedules (plan_sweep) and their memory on the device.
+// lists: the cells' lists where the caller has them; later: as in spare_memory.
 // Without the memory for them, or where a level is wider than the cluster's
 // signals can carry, the sweeps stay one launch per level.
-int build_chain(ofg_ctx *c, const NbLists *lists = nullptr) {
+int build_chain(ofg_ctx *c, const NbLists *lists = nullptr, size_t later = 0) {
     if (c->chain[0].lev) return OFG_OK;
     if (!c->chainStatus) {
         CK(cudaHostAlloc((void **)&c->chainStatus, sizeof(unsigned), cudaHostAllocDefault));
@@ -391,7 +392,7 @@ int build_chain(ofg_ctx *c, const NbLists *lists = nullptr) {
     }
     const size_t coef = n + whole((size_t)kChainCell * c->nCells * sizeof(double));
     const size_t bytes = coef + whole((size_t)std::max(plans[0].slots, plans[1].slots) * kEdgeCoefs * real);
-    if (!spare_memory(bytes)) return OFG_OK;
+    if (!spare_memory(bytes, later)) return OFG_OK;
     if (cudaMalloc((void **)&c->d_chain, bytes) != cudaSuccess) {
         cudaGetLastError();
         c->d_chain = nullptr;
@@ -655,9 +656,9 @@ int ofg_upload_mesh(ofg_ctx *c, int nNodes, const double *xN, const double *yN, 
     free_chain(c);
     if (c->d_gl[1]) { cudaFree(c->d_gl[1]); c->d_gl[1] = nullptr; }
     c->gl = 0;
-    NbLists L;
-    build_lists(c, L);
     {
+        NbLists L;   // given back here: kept to the end, the later host arrays took 15 ms more of 100 (312,500 cells)
+        build_lists(c, L);
         std::vector<int> lcb(c->lc.begin(), c->lc.begin() + nBFaces);
         if ((rc = upload(c, &c->d_lcb, lcb.data(), nBFaces))) return rc;
         if ((rc = upload(c, &c->d_nb_off, L.nbOff.data(), L.nbOff.size()))) return rc;
@@ -666,6 +667,9 @@ int ofg_upload_mesh(ofg_ctx *c, int nNodes, const double *xN, const double *yN, 
         if ((rc = upload(c, &c->d_lol, L.lol.data(), L.lol.size()))) return rc;
         if ((rc = upload(c, &c->d_up_off, L.upOff.data(), L.upOff.size()))) return rc;
         if ((rc = upload(c, &c->d_upl, L.upl.data(), L.upl.size()))) return rc;
+        if (!c->tuneSet) c->tune.sweep_persistent = chain_pays(c) ? 1 : 0;
+        if (c->tune.sweep_persistent && !multi_stage(c) && (rc = build_chain(c, &L, kCellBytes * nCells)))
+            return rc;
     }
     // metrics on the GPU (UnsGrid::CalcMetrics); for an SA solve without a
     // caller-supplied wall distance, CALC_WALL_DIST on the GPU as well
@@ -789,8 +793,6 @@ int ofg_upload_mesh(ofg_ctx *c, int nNodes, const double *xN, const double *yN, 
         CK(cudaMemset(c->d_dnut, 0, nT * sizeof(double)));
     }
     // what the solve can do without comes last
-    if (!c->tuneSet) c->tune.sweep_persistent = chain_pays(c) ? 1 : 0;
-    if (c->tune.sweep_persistent && !multi_stage(c) && (rc = build_chain(c, &L))) return rc;
     if (overlap_from(c) < INT_MAX && spare_memory(N * GLR * rs) &&
         cudaMalloc(&c->d_gl[1], N * GLR * rs) != cudaSuccess) {   // then the iterations do not overlap
         cudaGetLastError();
