@@ -1,8 +1,11 @@
 """The sweep schedule among a context's other choices: the autotuner times the
 level kernels' shapes with level launches whatever the context came with; a
 schedule that is not in use holds no memory; a second mesh uploaded into a
-context tuned to the chained sweeps.  The overlapped SA iteration of calls of ten and
-more: against whole iterations, and around a caller's stream."""
+context tuned to the chained sweeps; chained contexts made and dropped by several
+threads at once.  The overlapped SA iteration of calls of ten and more: against
+whole iterations, and around a caller's stream."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -121,3 +124,30 @@ def test_overlapped_calls_are_the_whole_iterations(order, precision, igrad):
             assert np.array_equal(a.field(field), b.field(field))
     assert np.array_equal(a.res_history(), b.res_history())
     batch.close()
+
+
+def test_chained_contexts_of_several_threads():
+    m, prm = meshgen.bump_channel(40, 20), P.euler_bump()
+
+    def solve():
+        s = Solver(m, prm)
+        s.init_flowfield()
+        s.step(3)
+        return s.state()
+
+    want, bad = solve(), []
+
+    def work():
+        try:
+            for _ in range(8):
+                if not np.array_equal(solve(), want):
+                    bad.append("different bits")
+        except Exception as e:
+            bad.append(e)
+
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
