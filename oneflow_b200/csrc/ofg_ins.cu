@@ -451,7 +451,7 @@ struct Gm {
     const double *A;
     const double *b;   // right-hand side
     double *x;         // solution
-    double *V;         // [kKrylov + 1][ld] normalised basis (ld: nT in whole 128 bytes, for the bulk copies)
+    double *V;         // [kKrylov + 1][ld] normalised basis (ld: nT in whole 128 bytes, for the tiles)
     size_t ld;
     double *W;         // [nT] unnormalised next vector
     double *Y;         // [nT] A v_j
@@ -698,11 +698,12 @@ __global__ void __launch_bounds__(kThreads, 3) k_gm_spmv_dots(Gm G, int j, const
     double *Vj = G.V + (size_t)j * G.ld;
     for (int r = threadIdx.x; r <= j; r += blockDim.x) acc[r] = 0.0;
     const int nChunks = (nT + kChunk - 1) / kChunk;
+    bool live = true;   // no wait of this warp has run out: after one that has, it copies nothing more
     for (int ch = blockIdx.x; ch < nChunks; ch += G.nChunkBlk) {
         const int r0 = ch * kChunk;
         // a pass's 8 KB come by one copy; the first one's ahead of the rows of A
         auto copy = [&](int rb) {
-            if (rb >= j || lane != 0) return;
+            if (!live || rb >= j || lane != 0) return;
             gm_expect(bar, 4 * kChunk * 8);
             gm_tile(mine, tiles, r0, rb, bar);
         };
@@ -730,12 +731,12 @@ __global__ void __launch_bounds__(kThreads, 3) k_gm_spmv_dots(Gm G, int j, const
         for (int k = 0; k < KR; ++k) yv[k] = ys[lane + 32 * k];
         // the stored basis vectors r < j, four per pass of the warp, each summed
         // over the lane's rows in ascending order, then over the warp; a pass's
-        // 8 KB come by bulk copies, the next pass's while this one's are summed
+        // 8 KB come as one tile, the next pass's while this one's are summed
         const double *ring0 = ring + (size_t)wid * 4 * kChunk;
-        for (int rb = first; rb < j; rb += G4) {
-            const bool ok = gm_wait(bar, phase);
+        for (int rb = first; live && rb < j; rb += G4) {
+            live = __all_sync(0xffffffffu, gm_wait(bar, phase));
             phase ^= 1;
-            if (!__all_sync(0xffffffffu, ok)) {
+            if (!live) {
                 S->timeout = 1;
                 gm_wait(bar, phase ^ 1);   // the copy in flight, once more
                 break;
@@ -846,11 +847,9 @@ __global__ void __launch_bounds__(kOrth + 32, 3) k_gm_orth(Gm G, int j, const __
                                 kOrthVec * p + q * kOrthBox, full + 8 * k);
                 }
             }
-        if (!ok) {
-            S->timeout = 1;
-            for (int q = max(0, n - kOrthRing); q < n; ++q)   // the copies in flight
-                gm_wait(full + 8 * (q % kOrthRing), (q / kOrthRing) & 1);
-        }
+        if (!ok) S->timeout = 1;
+        // the last copies, in flight still where a wait ran out, here or among their readers
+        for (int q = max(0, n - kOrthRing); q < n; ++q) gm_wait(full + 8 * (q % kOrthRing), (q / kOrthRing) & 1);
         return;
     }
     double v = 0.0;
