@@ -430,7 +430,7 @@ struct ofg_mlp {
     int pairs = 0;                     // pairs of blocks the device holds at once (0: not asked yet)
     MlpNet net{};
     bf16 *wf = nullptr, *wk = nullptr;
-    int capTiles = 0, capParts = 0;
+    int capTiles = 0;
     bf16 *Hf = nullptr, *dZf = nullptr;
     float *Gf = nullptr;
     long long adamStep = 0;

@@ -13,7 +13,8 @@
 //
 // The same products in the same order as layer-by-layer GEMMs (k_gemm): the
 // same bits.  Every wait is bounded; one that runs out sets g_gemm_status and
-// the block goes on without waiting, to the end.
+// the block goes on without waiting or fetching, to the end, where it waits (again
+// within the limit) for what it has in flight.
 //
 // Measured on the 22 -> 6 x 256 -> 4 network.  Prediction of 294,912 rows: 1.25 ms
 // with one tile a pair and cluster barriers (a stage of 10,500 cycles: 2,400
@@ -131,6 +132,15 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
         : "memory");
 }
 
+// After a wait that ran out, within the limit again: the thread's copies in flight
+// on the mbarriers full ..., whatever their phase, then its MMAs
+__device__ __noinline__ void mlp_drain(uint32_t full, int buffers) {
+    for (int k = 0; k < 2 * buffers + 2; ++k) {
+        if (k == 2 * buffers) mma_commit(full);
+        mbar_wait_cluster(full + 8 * (k / 2 % buffers), k & 1);
+    }
+}
+
 // where a pass's rows come from
 struct MlpRows {
     const float *x, *y;     // samples; y: targets (training), else null
@@ -240,9 +250,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FT + 32, 1) k_mlp_pa
                     const bool more = next < stages || (!TRAIN && t0 + NT * pairs < tiles);
                     if (more) {
                         wait(acc + 8 * behind, (seen[behind] - 1) & 1);
-                        fetch(next % stages, buf);
+                        if (__builtin_expect(ok, 1)) fetch(next % stages, buf);
                     }
                 }
+            if (__builtin_expect(!ok, 0)) mlp_drain(full, WB);
         }
         __syncwarp();
     } else {
@@ -520,7 +531,10 @@ __global__ void __launch_bounds__(DT, 3) k_mlp_dw(MlpNet P, DwGrid D, float *par
                 if (lane >= 16 && f < nt / 8) mlp_bulk(base + DW_STAGE / 2 + f * 2048, B + f * 1024, n * 16, full);
             }
             ok = __all_sync(0xffffffffu, mbar_wait(full, i & 1));
-            if (!ok) break;
+            if (!ok) {
+                mbar_wait(full, i & 1);   // the copies in flight, once more
+                break;
+            }
             if (lane == 0) {
                 tc_fence_after();
                 for (int j = 0; j < n / 16; ++j)
@@ -530,7 +544,10 @@ __global__ void __launch_bounds__(DT, 3) k_mlp_dw(MlpNet P, DwGrid D, float *par
             }
             __syncwarp();
             ok = __all_sync(0xffffffffu, mbar_wait(all, i & 1));   // before the next copies, and the results
-            if (!ok) break;
+            if (!ok) {
+                mbar_wait(all, i & 1);
+                break;
+            }
         }
         if (!ok && lane == 0) atomicOr(&g_gemm_status, 1u);
     }
