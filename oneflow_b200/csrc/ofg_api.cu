@@ -798,8 +798,7 @@ int ofg_upload_mesh(ofg_ctx *c, int nNodes, const double *xN, const double *yN, 
     if ((rc = upload<double>(c, &c->d_vissr, nullptr, N))) return rc;
     if ((rc = upload<double>(c, &c->d_rad, nullptr, N))) return rc;
     if ((rc = upload<double>(c, &c->d_bcq, nullptr, (size_t)std::max(nBFaces, 1) * NEQ))) return rc;
-    // (the gradient kernel's limiter extremes: 10 per block, blocks of 64 threads at the smallest)
-    c->nPartialMax = std::max<size_t>((N + 63) / 64 * 10, 2 * 148 * NEQ) + 16;
+    c->nPartialMax = (N + 127) / 128 * 2 * NEQ;   // k_res_max: a block's maxima and their cells
     if ((rc = upload<double>(c, &c->d_partial, nullptr, c->nPartialMax))) return rc;
     size_t nb128 = (N + 127) / 128;
     if ((rc = upload<double>(c, &c->d_npart, nullptr, nb128 * NEQ))) return rc;

@@ -210,6 +210,8 @@ __device__ __forceinline__ bool chain_wait(uint32_t bar, uint32_t parity) {
 // miss both and wait for a phase that waits for it.)
 template <bool CL, typename Body>
 __device__ __forceinline__ void chain_run(const ChainPlan &P, uint64_t *bars, double2 *word, Body &body) {
+    // a level's increments and words stay below what an mbarrier can count
+    static_assert(kChainLevel * Body::kBytes + 16 * kChainMaxBlocks < (1u << 20), "a level's bytes");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = CL ? chain_size() : 1, rank = CL ? chain_rank() : 0;
     const int g = warp / kChainWarps, w = warp % kChainWarps, cw = w * n + rank;

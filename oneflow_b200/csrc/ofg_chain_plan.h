@@ -16,7 +16,7 @@ constexpr int kChainWarps = 6, kChainGroups = 2, kChainThreads = 32 * kChainWarp
 // arrivals that a level's phase of a block's mbarrier waits for: one of every warp of its group (chain_run)
 constexpr int kChainArrivals = kChainWarps;
 constexpr int kChainRing = 4096, kChainMaxBlocks = 16;
-constexpr int kChainLevel = 16384;       // cells of a level: 64 bytes each stay below an mbarrier's 2^20 - 1
+constexpr int kChainLevel = 16384;      // most cells of a level: their bytes are counted on an mbarrier (chain_run)
 constexpr int kChainNone = INT32_MIN;   // an empty edge slot
 
 struct SweepPlan {

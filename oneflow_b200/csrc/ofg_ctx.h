@@ -38,7 +38,7 @@ struct ofg_ctx {
     // ---- device ----
     cudaStream_t stream = nullptr;      // stream every launch goes to
     cudaStream_t ownStream = nullptr;   // the context's own stream (set when a caller's stream is in use)
-    cudaStream_t sideStream = nullptr;  // the iteration graph's branch (capture only)
+    cudaStream_t sideStream = nullptr;  // the iteration's branch (kSteps), captured or as it stands
     cudaEvent_t forkEvent[2] = {nullptr, nullptr};
     int *d_lcb = nullptr, *d_bct = nullptr;                 // left cell and BC code of each boundary face
     int *d_nb_off = nullptr, *d_nbl = nullptr;              // per-cell neighbour lists (int2 pairs)
@@ -48,7 +48,7 @@ struct ofg_ctx {
     char *d_chain = nullptr;                                // their memory
     void *d_chainCoef = nullptr;                            // edge coefficients of the sweep under way
     double *d_chainCell = nullptr;                          // and its cells' values, in the sweep's order
-    unsigned *chainStatus = nullptr;                        // pinned: a chained sweep's wait ran out
+    unsigned *chainStatus = nullptr;                        // pinned (StatusWords): a chained sweep's wait ran out
     bool tuneSet = false;                                   // launch shapes chosen by the caller or the autotuner
     void *d_fgeo = nullptr, *d_cgeo = nullptr;              // face / cell records at the face precision
     double *d_fgeoD = nullptr;                              // mixed path: FP64 face records

@@ -297,7 +297,7 @@ def run_experiment(n_train: int = 192, n_test: int = 32, width: int = 256, depth
 
     out = {"family": fam.description,
            "features": list(fam.feature_names),
-           "network": f"{X.shape[1]}->{depth}x{width} GELU->{Y.shape[1]}, BF16 tcgen05.mma GEMMs",
+           "network": f"{X.shape[1]}->{depth}x{width} GELU->{Y.shape[1]}, BF16 tcgen05.mma",
            "train_cases": n_train, "train_cases_converged": int(sum(i is not None for i in train_iters)),
            "test_cases": n_test, "train_samples": int(X.shape[0]),
            "train_steps": train_steps, "batch": batch, "lr": lr,
