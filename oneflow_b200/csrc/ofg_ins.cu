@@ -811,7 +811,7 @@ __global__ void __launch_bounds__(kThreads) k_gm_hsum(Gm G, int j) {
 // of 16,900 / 65,800 rows: 13.7 / 34.8 with 32 loads a thread ahead; 14.7 / 30.9 with
 // a copy a vector (an SM takes some 75 cycles for each, however small) and
 // eight vectors a stage; 10.8 / 26.2 with 32; 6.4 / 23.2 with tiles of 16 vectors
-// by one TMA instruction, 0.87 of the measured HBM rate at the larger size.
+// by one TMA instruction: 5.7 TB/s of basis at the larger size, part of it from L2.
 __global__ void __launch_bounds__(kOrth + 32, 3) k_gm_orth(Gm G, int j, const __grid_constant__ CUtensorMap tiles) {
     extern __shared__ __align__(128) double ring[];   // [kOrthRing][kOrthVec][kOrth]
     __shared__ double hcol[kHCol];
