@@ -20,8 +20,8 @@
 // bits.  Every wait is bounded; one that runs out raises *status.
 //
 // Measured, us a sweep (level launches / chained): 385 levels of 170 cells,
-// FP64, 3,130 / 430; 119 of 29 cells 785-950 / 83.  What bounds a level now
-// (0.7 us alone, 1.1 us in a cluster of 4) is the arithmetic of its cells: about
+// FP64, 3,130 / 400; 119 of 29 cells 785-950 / 80.  What bounds a level now
+// (0.66 us alone, 1.03 us in a cluster of 4) is the arithmetic of its cells: about
 // 160 FP64 instructions a cell at 2.4 cycles a warp, their 9-cycle latencies
 // and the signal (0.06 us in a block, 0.25 us in a cluster).  Two groups of six
 // warps: the loads of a level (0.5 us) end before its wait does, and 168
